@@ -98,6 +98,10 @@ void attach_factors(cruna_ctx *c, LineOp &op, const HostFactors &hf) {
     op.fbnorm = upload(c, hf.fbnorm);
     op.fbrat = hf.fbrat;
   }
+  std::vector<double> tab;
+  if (build_line_table(op.n, hf.raw_dl, hf.raw_d, hf.raw_du, op.cyclic ? hf.fbnorm : std::vector<double>(), tab, op.kf,
+                       op.kb))
+    op.tab = upload(c, tab);
 }
 
 long long N5(const cruna_ctx *c) { return c->g.N * 5; }
@@ -138,7 +142,7 @@ double *rhs_buffer(cruna_ctx *c) {
 
 // time_stepper_direct (rk_o4_e.f90:17-58): q1 may alias q0
 void step_direct(cruna_ctx *c, const double *q0, double *q1) {
-  double *k = (use_fused(c) && !c->has_rhs_bc) ? nullptr : rhs_buffer(c);
+  double *k = ((use_fused(c) || c->dir_ok) && !c->has_rhs_bc) ? nullptr : rhs_buffer(c);
   double *acc = c->st[1], *qa = c->st[2], *qb = c->st[3], *qbc = c->st[4];
   const double dt = c->cfg.dt;
   if (use_fused(c)) {
@@ -159,25 +163,21 @@ void step_direct(cruna_ctx *c, const double *q0, double *q1) {
   ensure_generic(c);
   halo(c, q0, 5);
   closure_stage(c, q0);
-  rhs_direct_generic(c, q0, k, qbc);
-  rk_stage(c, 1, dt, k, q0, acc, qa);
+  stage_direct_generic(c, q0, k, qbc, 1, q0, acc, qa, dt);
   halo(c, qa, 5);
   closure_stage(c, qa);
-  rhs_direct_generic(c, qa, k, qbc);
-  rk_stage(c, 2, dt, k, q0, acc, qb);
+  stage_direct_generic(c, qa, k, qbc, 2, q0, acc, qb, dt);
   halo(c, qb, 5);
   closure_stage(c, qb);
-  rhs_direct_generic(c, qb, k, qbc);
-  rk_stage(c, 3, dt, k, q0, acc, qa);
+  stage_direct_generic(c, qb, k, qbc, 3, q0, acc, qa, dt);
   halo(c, qa, 5);
   closure_stage(c, qa);
-  rhs_direct_generic(c, qa, k, qbc);
-  rk_stage(c, 4, dt, k, q0, acc, q1);
+  stage_direct_generic(c, qa, k, qbc, 4, q0, acc, q1, dt);
 }
 
 // time_stepper_adjoint (rk_o4_e.f90:62-105): dt -> -dt, q0 frozen; qs1 may alias qs0
 void step_adjoint(cruna_ctx *c, const double *qs0, const double *q0, const double *g, double *qs1) {
-  double *k = (use_fused(c) && !c->has_rhs_bc) ? nullptr : rhs_buffer(c);
+  double *k = ((use_fused(c) || c->dir_ok) && !c->has_rhs_bc) ? nullptr : rhs_buffer(c);
   double *acc = c->st[1], *qa = c->st[2], *qb = c->st[3], *qbc = c->st[4];
   const double dt = -c->cfg.dt;
   halo(c, q0, 5);
@@ -194,17 +194,13 @@ void step_adjoint(cruna_ctx *c, const double *qs0, const double *q0, const doubl
   }
   ensure_generic(c);
   halo(c, qs0, 5);
-  rhs_adjoint_generic(c, qs0, q0, g, k, qbc);
-  rk_stage(c, 1, dt, k, qs0, acc, qa);
+  stage_adjoint_generic(c, qs0, q0, g, k, qbc, 1, qs0, acc, qa, dt);
   halo(c, qa, 5);
-  rhs_adjoint_generic(c, qa, q0, g, k, qbc);
-  rk_stage(c, 2, dt, k, qs0, acc, qb);
+  stage_adjoint_generic(c, qa, q0, g, k, qbc, 2, qs0, acc, qb, dt);
   halo(c, qb, 5);
-  rhs_adjoint_generic(c, qb, q0, g, k, qbc);
-  rk_stage(c, 3, dt, k, qs0, acc, qa);
+  stage_adjoint_generic(c, qb, q0, g, k, qbc, 3, qs0, acc, qa, dt);
   halo(c, qa, 5);
-  rhs_adjoint_generic(c, qa, q0, g, k, qbc);
-  rk_stage(c, 4, dt, k, qs0, acc, qs1);
+  stage_adjoint_generic(c, qa, q0, g, k, qbc, 4, qs0, acc, qs1, dt);
 }
 
 bool due(int freq, int nt) { return freq > 0 && nt % freq == 0; }
@@ -492,6 +488,8 @@ int cruna_init(const cruna_config *cfg, const double *bc_table, int nbc, cruna_c
     c->flag = static_cast<int *>(fl);  // [0] state check, [1] a kernel's bounded wait ran out
     CRUNA_CUDA_CHECK(cudaMemsetAsync(fl, 0, sizeof(int) * 4, c->stream));
     c->fused_ok = fused_supported(c);
+    c->dir_ok = dir_passes_supported(c);
+    c->march_y_ok = march_y_supported(c);
     c->filter_fused_ok = filter_fused_supported(c);
     CRUNA_CUDA_CHECK(cudaStreamSynchronize(c->stream));
     return CRUNA_OK;

@@ -20,6 +20,8 @@ namespace cruna {
 constexpr int kMaxR = 6;        // largest interior half-width (o10 filter: 5)
 constexpr int kMaxRows = 5;     // largest number of explicit boundary rows at one end
 constexpr int kMaxRowW = 12;    // widest boundary row (o10 filter: 11 points)
+constexpr int kLineL = 16;      // points of a line held by one thread of the line engine (lines.cuh)
+constexpr int kLineMaxN = 2048; // longest line of the line engine: its row table takes 48 n bytes of shared memory
 
 enum OpKind { OP_ZERO = 0, OP_COPY = 1, OP_STENCIL = 2 };
 
@@ -47,6 +49,10 @@ struct LineOp {
   // device factor arrays (owned by the context)
   const double *dl = nullptr, *inv_d = nullptr, *du = nullptr, *du2 = nullptr, *fbnorm = nullptr;
   const int *ipiv = nullptr;
+  // row table of the line engine (lines.cuh), or null: 6 doubles a row (l, Pf, 1/u, c, Qb, fbnorm), rows padded
+  // to a multiple of kLineL; kf, kb: chunks a sweep looks back (forward / backward)
+  const double *tab = nullptr;
+  int kf = 0, kb = 0;
 };
 
 // Host-side copy of the factors (filled by the dgttrf restatement in schemes.cpp).
@@ -85,6 +91,11 @@ bool diff_is_periodic(int scheme);
 int lapack_dgttrf(int n, double *dl, double *d, double *du, double *du2, int *ipiv);
 void lapack_dgttrs(int n, const double *dl, const double *d, const double *du, const double *du2,
                    const int *ipiv, double *b);
+
+// row table of the line engine for the tridiagonal matrix (dl, d, du), factored without row interchanges;
+// fbnorm: the cyclic correction's vector or empty.  False when a pivot is too small for that.
+bool build_line_table(int n, const std::vector<double> &dl, const std::vector<double> &d, const std::vector<double> &du,
+                      const std::vector<double> &fbnorm, std::vector<double> &tab, int &kf, int &kb);
 
 // error raised inside the library and returned by the extern "C" entry points as (code, message)
 struct ApiError {
@@ -126,6 +137,8 @@ struct cruna_ctx {
   std::string err;
   bool force_generic = false;
   bool fused_ok = false;
+  bool dir_ok = false;          // generic path on the per-direction passes (dir_passes.cu)
+  bool march_y_ok = false;      // generic path: x and z marching, y on the line engine (fused.cu)
   bool tma_fused = false;       // FP64 adjoint pass fed by TMA where the layout allows (cruna_set_tma_passes)
   bool filter_fused_ok = false;
   // FP32-stencil path: pressure / temperature offsets differenced in FP32 (set once per context)
@@ -199,6 +212,29 @@ void rhs_direct_generic(cruna_ctx *c, const double *q, double *rhs, double *qbc_
 void generic_forward_gradients(cruna_ctx *c, const double *q);  // primitives, grads, mu, tau into tmp
 void rhs_adjoint_generic(cruna_ctx *c, const double *qs, const double *q, const double *g, double *rhs,
                          double *qsbc_scratch);
+// the same RHS (stage 0) or RK stage on per-direction passes (dir_passes.cu), where they apply
+bool dir_passes_supported(const cruna_ctx *c);
+void rhs_direct_dir(cruna_ctx *c, const double *q, double *rhs, double *qbc_scratch, int bc_mask, int stage,
+                    const double *q0, double *acc, double *qnext, double dt);
+void rhs_adjoint_dir(cruna_ctx *c, const double *qs, const double *q, const double *g, double *rhs,
+                     double *qsbc_scratch, int stage, const double *qs0, double *acc, double *qnext, double dt);
+bool only_sponge(const cruna_ctx *c);  // the RHS boundary table is one type-400 row
+// one direction's pass: gradients (slots F_UX + d, ...) and convective accumulators; stresses' and heat flux's
+// divergence onto r[1..4]; adjoint terms
+void dir_flux(cruna_ctx *c, int d, const double *q, double *t, double *r, bool first);
+void dir_viscous(cruna_ctx *c, int d, const double *t1, const double *t2, const double *t3, const double *h, double *r);
+void dir_adjoint(cruna_ctx *c, int d, const double *qs, const double *q, double *r, bool first);
+// x and z in the z-marching passes, y on the line engine (fused.cu, fused_adjoint.cu)
+bool march_y_supported(const cruna_ctx *c);
+void rhs_direct_march_y(cruna_ctx *c, const double *q, double *rhs, double *qbc_scratch, int bc_mask, int stage,
+                        const double *q0, double *acc, double *qnext, double dt);
+void rhs_adjoint_march_y(cruna_ctx *c, const double *qs, const double *q, const double *g, double *rhs,
+                         double *qsbc_scratch, int stage, const double *qs0, double *acc, double *qnext, double dt);
+// one RK stage of the generic path: its RHS and the stage update
+void stage_direct_generic(cruna_ctx *c, const double *q, double *k, double *qbc_scratch, int stage, const double *q0,
+                          double *acc, double *qnext, double dt);
+void stage_adjoint_generic(cruna_ctx *c, const double *qs, const double *q, const double *g, double *k,
+                           double *qsbc_scratch, int stage, const double *qs0, double *acc, double *qnext, double dt);
 bool fused_supported(const cruna_ctx *c);
 void rhs_direct_fused(cruna_ctx *c, const double *q, double *rhs, int stage, const double *q0,
                       double *acc, double *qnext, double dt);

@@ -120,6 +120,9 @@ void build_transpose(cruna_ctx *c, const LineOp &op, const HostFactors &hf, Line
   for (size_t i = 0; i < ht.d.size(); ++i) inv[i] = 1.0 / ht.d[i];
   t.sop = op;
   t.sop.cyclic = 0;
+  t.sop.tab = nullptr;
+  std::vector<double> tab;
+  if (build_line_table(n, hf.raw_du, hf.raw_d, hf.raw_dl, {}, tab, t.sop.kf, t.sop.kb)) t.sop.tab = upload_vec(c, tab);
   t.sop.dl = upload_vec(c, ht.dl);
   t.sop.inv_d = upload_vec(c, inv);
   t.sop.du = upload_vec(c, ht.du);
@@ -723,15 +726,11 @@ void step_direct_vjp(cruna_ctx *c, const double *q0, const double *lam1, double 
     rhs_direct_fused(c, S[S_Q3], k, 3, q0, acc, S[S_Q4], dt);
     if (need_q1) rhs_direct_fused(c, S[S_Q4], k, 4, q0, acc, S[S_Q1], dt);
   } else {
-    rhs_direct_generic(c, q0, k, c->st[4]);
-    rk_stage(c, 1, dt, k, q0, acc, S[S_Q2]);
-    rhs_direct_generic(c, S[S_Q2], k, c->st[4]);
-    rk_stage(c, 2, dt, k, q0, acc, S[S_Q3]);
-    rhs_direct_generic(c, S[S_Q3], k, c->st[4]);
-    rk_stage(c, 3, dt, k, q0, acc, S[S_Q4]);
+    stage_direct_generic(c, q0, k, c->st[4], 1, q0, acc, S[S_Q2], dt);
+    stage_direct_generic(c, S[S_Q2], k, c->st[4], 2, q0, acc, S[S_Q3], dt);
+    stage_direct_generic(c, S[S_Q3], k, c->st[4], 3, q0, acc, S[S_Q4], dt);
     if (need_q1) {
-      rhs_direct_generic(c, S[S_Q4], k, c->st[4]);
-      rk_stage(c, 4, dt, k, q0, acc, S[S_Q1]);
+      stage_direct_generic(c, S[S_Q4], k, c->st[4], 4, q0, acc, S[S_Q1], dt);
     }
   }
   // reverse: filters i3, i2, i1, then the BC on q outside the RHS (computation_direct.f90:76-100)

@@ -23,6 +23,7 @@
 
 #include "cruna_internal.cuh"
 #include "fused_common.cuh"
+#include "ops_common.cuh"
 
 namespace cruna {
 
@@ -56,14 +57,18 @@ constexpr size_t cl_offset_g() { return ((plane_bytes_g<T, R>() + ring_bytes_g<T
 template <typename T, int R>
 constexpr bool cl_alias_plane() { return plane_bytes_g<T, R>() >= kClActBytes; }
 
-template <typename T, int R, bool PER, bool CL = false>
+//
+// YX: the y derivatives come from the line engine (compact schemes along y, dir_passes.cu): the tile has no y
+// halos and the pass adds a.yr and reads the gradients of a.yt.
+template <typename T, int R, bool PER, bool CL = false, bool YX = false>
 __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const __grid_constant__ FusedArgs a) {
-  constexpr int PW = TX + 2 * R, PH = TY + 2 * R, PS = PW * PH;
+  constexpr int RY = YX ? 0 : R, NPF = YX ? 6 : 7;
+  constexpr int PW = TX + 2 * R, PH = TY + 2 * RY, PS = PW * PH;
   constexpr int NS = ring_slots(R);
   constexpr int NRF = 6, RS = TX * TY;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  T *plane = reinterpret_cast<T *>(smem_raw);          // [7][PH][PW]
-  T *ring = plane + 7 * PS;                            // [NS][NRF][TY*TX]
+  T *plane = reinterpret_cast<T *>(smem_raw);          // [NPF][PH][PW]
+  T *ring = plane + NPF * PS;                          // [NS][NRF][TY*TX]
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
   const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
   const int k0 = blockIdx.z * a.kc;
@@ -76,7 +81,7 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const
   const int colpt = gi + n1 * gj;
   const long long N = a.g.N;
   const double *Q0 = a.q, *Q1 = a.q + N, *Q2 = a.q + 2 * N, *Q3 = a.q + 3 * N, *Q4 = a.q + 4 * N;
-  HaloSet<R> hs;
+  HaloSet<R, RY> hs;
   hs.init(ox, oy, i0, j0, tid, n1);
   // closure: weights staged once per block, TMEM for the three products (128 lanes x 128 columns)
   ClSmem *cs = nullptr;
@@ -132,12 +137,12 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const
     if (col && kc < k1) {
       const long long pt = colpt + (long long)n12 * kc;
       pruv[0] = Q1[pt];
-      pruv[1] = Q2[pt];
+      if constexpr (!YX) pruv[1] = Q2[pt];
     }
   };
   prefetch(k0 + R, k0);
   // raw state of this thread's halo cells, loaded one plane ahead
-  constexpr int NHT = HaloSet<R>::PER_THREAD;
+  constexpr int NHT = HaloSet<R, RY>::PER_THREAD;
   double hv[NHT][5];
   auto halo_fetch = [&](int kk) {
     const long long kofs = (long long)n12 * kk;
@@ -156,12 +161,12 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const
     if (pf_ok) put_ring(k + R, pf[0], pf[1], pf[2], pf[3], pf[4]);
     const int slot = k % NS;
     {
-      T *c = plane + (ty + R) * PW + (tx + R);
+      T *c = plane + (ty + RY) * PW + (tx + R);
       const T *rp = ring + slot * NRF * RS + tid;
 #pragma unroll
       for (int f = 0; f < 5; ++f) c[f * PS] = rp[f * RS];
       c[5 * PS] = T(pruv[0]);
-      c[6 * PS] = T(pruv[1]);
+      if constexpr (!YX) c[6 * PS] = T(pruv[1]);
     }
     const long long kofs = (long long)n12 * k;
 #pragma unroll
@@ -172,14 +177,27 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const
       T *c = plane + hs.cell[h];
       c[0 * PS] = T(ru * ir); c[1 * PS] = T(rv * ir); c[2 * PS] = T(rw * ir);
       c[3 * PS] = T(a.WoR * p * ir - a.T_ref);
-      c[4 * PS] = T(p - a.p_ref); c[5 * PS] = T(ru); c[6 * PS] = T(rv);
+      c[4 * PS] = T(p - a.p_ref); c[5 * PS] = T(ru);
+      if constexpr (!YX) c[6 * PS] = T(rv);
     }
     prefetch(k + R + 1, k + 1);
     if (k + 1 < k1) halo_fetch(k + 1);
+    double yd[YX ? 9 : 1];                             // u_y, v_y, w_y, T_y and the y part of the convective terms
+    if constexpr (YX) {
+      if (inside) {
+        const long long pt = colpt + kofs;
+        yd[0] = a.yt[pt + F_UY * N];
+        yd[1] = a.yt[pt + F_VY * N];
+        yd[2] = a.yt[pt + F_WY * N];
+        yd[3] = a.yt[pt + F_TY * N];
+#pragma unroll
+        for (int v = 0; v < 5; ++v) yd[4 + v] = a.yr[pt + v * N];
+      }
+    }
     __syncthreads();
     if (inside) {
       const int i = i0 + tx, j = j0 + ty;
-      const T *c = plane + (ty + R) * PW + (tx + R);
+      const T *c = plane + (ty + RY) * PW + (tx + R);
       const T *U = c, *V = c + PS, *W = c + 2 * PS, *TT = c + 3 * PS, *P = c + 4 * PS, *RU = c + 5 * PS,
               *RV = c + 6 * PS;
       int so[NS];
@@ -213,11 +231,21 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const
       const T ezp = Dz2<T, R, PER>(oz, zt, zw, k) * sz;
       const T wc = zw[R];
       // velocity gradients (ns_rho_rhou_p.f90:102-112) and temperature gradient (:189-191)
-      const T ux = D1<T, R, PER>(ox, U, 1, i) * sx, uy = D1<T, R, PER>(oy, U, PW, j) * sy;
-      const T vx = D1<T, R, PER>(ox, V, 1, i) * sx, vy = D1<T, R, PER>(oy, V, PW, j) * sy;
-      const T wx = D1<T, R, PER>(ox, W, 1, i) * sx, wy = D1<T, R, PER>(oy, W, PW, j) * sy;
+      const T ux = D1<T, R, PER>(ox, U, 1, i) * sx, vx = D1<T, R, PER>(ox, V, 1, i) * sx;
+      const T wx = D1<T, R, PER>(ox, W, 1, i) * sx;
       const T tgx = D1<T, R, PER>(ox, TT, 1, i) * T(ox.scale_h);
-      const T tgy = D1<T, R, PER>(oy, TT, PW, j) * T(oy.scale_h);
+      T uy, vy, wy, tgy;
+      if constexpr (YX) {
+        uy = T(yd[0]);
+        vy = T(yd[1]);
+        wy = T(yd[2]);
+        tgy = T(yd[3]);
+      } else {
+        uy = D1<T, R, PER>(oy, U, PW, j) * sy;
+        vy = D1<T, R, PER>(oy, V, PW, j) * sy;
+        wy = D1<T, R, PER>(oy, W, PW, j) * sy;
+        tgy = D1<T, R, PER>(oy, TT, PW, j) * T(oy.scale_h);
+      }
       // viscosity mu0 (T/T0)^1.5 (T0+S1)/(T+S1) and stresses (:115-128); x^1.5 as x*sqrt(x)
       const double Tabs = double(Tc) + a.T_ref;
       const double tr = Tabs / a.T0;
@@ -233,22 +261,34 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const
       const T phi = t11 * ux + t12 * uy + t13 * uz + t12 * vx + t22 * vy + t23 * vz + t13 * wx + t23 * wy +
                     t33 * wz;                                     // :204-206
       // convective terms (:131-186)
-      const T m1 = D1<T, R, PER>(ox, RU, 1, i) * sx, m2 = D1<T, R, PER>(oy, RV, PW, j) * sy;
-      const T px = D1<T, R, PER>(ox, P, 1, i) * sx, py = D1<T, R, PER>(oy, P, PW, j) * sy;
-      const T a1x = D2<T, R, PER>(ox, RU, U, 1, i) * sx, a1y = D2<T, R, PER>(oy, RV, U, PW, j) * sy;
-      const T a2x = D2<T, R, PER>(ox, RU, V, 1, i) * sx, a2y = D2<T, R, PER>(oy, RV, V, PW, j) * sy;
-      const T a3x = D2<T, R, PER>(ox, RU, W, 1, i) * sx, a3y = D2<T, R, PER>(oy, RV, W, PW, j) * sy;
+      const T m1 = D1<T, R, PER>(ox, RU, 1, i) * sx;
+      const T px = D1<T, R, PER>(ox, P, 1, i) * sx;
+      const T a1x = D2<T, R, PER>(ox, RU, U, 1, i) * sx, a2x = D2<T, R, PER>(ox, RU, V, 1, i) * sx;
+      const T a3x = D2<T, R, PER>(ox, RU, W, 1, i) * sx;
       const T pref = T(a.p_ref);
       const T ex = pref * ux + D2<T, R, PER>(ox, P, U, 1, i) * sx;
-      const T ey = pref * vy + D2<T, R, PER>(oy, P, V, PW, j) * sy;
       const T ez = pref * wz + ezp;
       const double gt = a.gamma / (a.gamma - 1.0);
-      const T c1 = -m1 - m2 - m3;
-      const T c2 = -a1x - a1y - a1z - px;
-      const T c3 = -a2x - a2y - a2z - py;
-      const T c4 = -a3x - a3y - a3z - pz;
-      T c5 = T(gt) * (-ex - ey - ez);
-      c5 = c5 + uc * px + vc * py + wc * pz;
+      T c1, c2, c3, c4, c5;
+      if constexpr (YX) {
+        c1 = T(yd[4]) - m1 - m3;
+        c2 = T(yd[5]) - a1x - a1z - px;
+        c3 = T(yd[6]) - a2x - a2z;
+        c4 = T(yd[7]) - a3x - a3z - pz;
+        c5 = T(yd[8]) + T(gt) * (-ex - ez);
+        c5 = c5 + uc * px + wc * pz;
+      } else {
+        const T m2 = D1<T, R, PER>(oy, RV, PW, j) * sy, py = D1<T, R, PER>(oy, P, PW, j) * sy;
+        const T a1y = D2<T, R, PER>(oy, RV, U, PW, j) * sy, a2y = D2<T, R, PER>(oy, RV, V, PW, j) * sy;
+        const T a3y = D2<T, R, PER>(oy, RV, W, PW, j) * sy;
+        const T ey = pref * vy + D2<T, R, PER>(oy, P, V, PW, j) * sy;
+        c1 = -m1 - m2 - m3;
+        c2 = -a1x - a1y - a1z - px;
+        c3 = -a2x - a2y - a2z - py;
+        c4 = -a3x - a3y - a3z - pz;
+        c5 = T(gt) * (-ex - ey - ez);
+        c5 = c5 + uc * px + vc * py + wc * pz;
+      }
       const T o[NG] = {c1, c2, c3, c4, c5, t11, t12, t13, t22, t23, t33, lam * tgx, lam * tgy, lam * tgz, phi};
       if constexpr (CL) {
 #pragma unroll
@@ -358,14 +398,17 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const
 // pass D
 // plane fields: 0 t11, 1 t12, 2 t13, 3 t22, 4 t23, 5 hx, 6 hy ; ring fields: 0 t13, 1 t23, 2 t33, 3 hz
 // ------------------------------------------------------------------------------------------------
-template <typename T, int R, bool PER>
+// YX: without the y derivatives, which the line engine has added to the convective terms already (plane fields
+// 0 t11, 1 t12, 2 t13, 3 hx, no y halos)
+template <typename T, int R, bool PER, bool YX = false>
 __global__ void __launch_bounds__(TX *TY, 3) k_pass_d(const __grid_constant__ FusedArgs a) {
-  constexpr int PW = TX + 2 * R, PH = TY + 2 * R, PS = PW * PH;
+  constexpr int RY = YX ? 0 : R, NPF = YX ? 4 : 7;
+  constexpr int PW = TX + 2 * R, PH = TY + 2 * RY, PS = PW * PH;
   constexpr int NS = ring_slots(R);
   constexpr int NRF = 4, RS = TX * TY;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  T *plane = reinterpret_cast<T *>(smem_raw);          // [7][PH][PW]
-  T *ring = plane + 7 * PS;                            // [NS][NRF][TY*TX]
+  T *plane = reinterpret_cast<T *>(smem_raw);          // [NPF][PH][PW]
+  T *ring = plane + NPF * PS;                          // [NS][NRF][TY*TX]
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
   const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
   const int k0 = blockIdx.z * a.kc;
@@ -378,9 +421,9 @@ __global__ void __launch_bounds__(TX *TY, 3) k_pass_d(const __grid_constant__ Fu
   const bool col = gi >= 0 && gj >= 0;
   const int colpt = gi + n1 * gj;
   const T *G = static_cast<const T *>(a.gbuf);
-  constexpr int pfld[7] = {5, 6, 7, 8, 9, 11, 12};   // G fields of the plane
+  constexpr int pfld[7] = {5, 6, 7, YX ? 11 : 8, 9, 11, 12};   // G fields of the plane (the first NPF)
   constexpr int rfld[4] = {7, 9, 10, 13};            // G fields of the ring
-  HaloSet<R> hs;
+  HaloSet<R, RY> hs;
   hs.init(ox, oy, i0, j0, tid, n1);
 
   for (int kk = k0 - R; kk < k0 + R; ++kk) {
@@ -392,7 +435,7 @@ __global__ void __launch_bounds__(TX *TY, 3) k_pass_d(const __grid_constant__ Fu
     for (int f = 0; f < NRF; ++f) rp[f * RS] = G[pt + rfld[f] * N];
   }
   T pf[NRF];
-  T pc[7];
+  T pc[NPF];
   int pf_ok = 0;
   auto prefetch = [&](int kk, int kc) {
     const int gk = gidx(oz, kk);
@@ -405,12 +448,12 @@ __global__ void __launch_bounds__(TX *TY, 3) k_pass_d(const __grid_constant__ Fu
     if (col && kc < k1) {
       const long long pt = colpt + (long long)n12 * kc;
 #pragma unroll
-      for (int f = 0; f < 7; ++f) pc[f] = G[pt + pfld[f] * N];
+      for (int f = 0; f < NPF; ++f) pc[f] = G[pt + pfld[f] * N];
     }
   };
   prefetch(k0 + R, k0);
-  constexpr int NHT = HaloSet<R>::PER_THREAD;
-  T hv[NHT][7];
+  constexpr int NHT = HaloSet<R, RY>::PER_THREAD;
+  T hv[NHT][NPF];
   auto halo_fetch = [&](int kk) {
     const long long kofs = (long long)n12 * kk;
 #pragma unroll
@@ -418,7 +461,7 @@ __global__ void __launch_bounds__(TX *TY, 3) k_pass_d(const __grid_constant__ Fu
       if (hs.goff[h] < 0) continue;
       const long long pt = hs.goff[h] + kofs;
 #pragma unroll
-      for (int f = 0; f < 7; ++f) hv[h][f] = G[pt + pfld[f] * N];
+      for (int f = 0; f < NPF; ++f) hv[h][f] = G[pt + pfld[f] * N];
     }
   };
   halo_fetch(k0);
@@ -430,9 +473,9 @@ __global__ void __launch_bounds__(TX *TY, 3) k_pass_d(const __grid_constant__ Fu
     }
     const int slot = k % NS;
     {
-      T *c = plane + (ty + R) * PW + (tx + R);
+      T *c = plane + (ty + RY) * PW + (tx + R);
 #pragma unroll
-      for (int f = 0; f < 7; ++f) c[f * PS] = pc[f];
+      for (int f = 0; f < NPF; ++f) c[f * PS] = pc[f];
     }
     const long long kofs = (long long)n12 * k;
     // epilogue inputs of this plane, issued before the barrier so their latency overlaps the stencils
@@ -461,14 +504,14 @@ __global__ void __launch_bounds__(TX *TY, 3) k_pass_d(const __grid_constant__ Fu
       if (hs.goff[h] < 0) continue;
       T *c = plane + hs.cell[h];
 #pragma unroll
-      for (int f = 0; f < 7; ++f) c[f * PS] = hv[h][f];
+      for (int f = 0; f < NPF; ++f) c[f * PS] = hv[h][f];
     }
     prefetch(k + R + 1, k + 1);
     if (k + 1 < k1) halo_fetch(k + 1);
     __syncthreads();
     if (inside) {
       const int i = i0 + tx, j = j0 + ty;
-      const T *c = plane + (ty + R) * PW + (tx + R);
+      const T *c = plane + (ty + RY) * PW + (tx + R);
       int so[NS];
 #pragma unroll
       for (int m = -R; m <= R; ++m) so[m + R] = ((slot + m + NS) % NS) * NRF * RS + tid;
@@ -487,13 +530,16 @@ __global__ void __launch_bounds__(TX *TY, 3) k_pass_d(const __grid_constant__ Fu
       for (int m = 0; m < NS; ++m) zc[m] = ring[so[m] + 3 * RS];
       const T qz = Dz1<T, R, PER>(oz, zc, k) * T(oz.scale_h);     // d_z (lambda d_z T)
       const T v1x = D1<T, R, PER>(ox, c + 0 * PS, 1, i) * sx;     // d_x tau_11
-      const T v1y = D1<T, R, PER>(oy, c + 1 * PS, PW, j) * sy;    // d_y tau_12
       const T v2x = D1<T, R, PER>(ox, c + 1 * PS, 1, i) * sx;     // d_x tau_21
-      const T v2y = D1<T, R, PER>(oy, c + 3 * PS, PW, j) * sy;    // d_y tau_22
       const T v3x = D1<T, R, PER>(ox, c + 2 * PS, 1, i) * sx;     // d_x tau_31
-      const T v3y = D1<T, R, PER>(oy, c + 4 * PS, PW, j) * sy;    // d_y tau_32
-      const T qx = D1<T, R, PER>(ox, c + 5 * PS, 1, i) * T(ox.scale_h);
-      const T qy = D1<T, R, PER>(oy, c + 6 * PS, PW, j) * T(oy.scale_h);
+      const T qx = D1<T, R, PER>(ox, c + (YX ? 3 : 5) * PS, 1, i) * T(ox.scale_h);
+      T v1y = T(0), v2y = T(0), v3y = T(0), qy = T(0);
+      if constexpr (!YX) {
+        v1y = D1<T, R, PER>(oy, c + 1 * PS, PW, j) * sy;          // d_y tau_12
+        v2y = D1<T, R, PER>(oy, c + 3 * PS, PW, j) * sy;          // d_y tau_22
+        v3y = D1<T, R, PER>(oy, c + 4 * PS, PW, j) * sy;          // d_y tau_32
+        qy = D1<T, R, PER>(oy, c + 6 * PS, PW, j) * T(oy.scale_h);
+      }
       const long long pt = opt;
       (void)i; (void)j;
       // assembly in the reference's order (:135, 143-149, 157-163, 171-177, 185-209)
@@ -511,7 +557,16 @@ __global__ void __launch_bounds__(TX *TY, 3) k_pass_d(const __grid_constant__ Fu
       if (a.force) {                                              // :212
         r1 = r1 + e_f[0]; r2 = r2 + e_f[1]; r3 = r3 + e_f[2]; r4 = r4 + e_f[3]; r5 = r5 + e_f[4];
       }
-      const double kv[5] = {r1, r2, r3, r4, r5};
+      double kv[5] = {r1, r2, r3, r4, r5};
+      if constexpr (YX) {
+        if (a.sp_qref) {                                          // type-400 sponge (:218)
+          const double sh = sponge_at(a.sponge, a.g, opt);
+          if (sh != 0.0) {
+#pragma unroll
+            for (int v = 0; v < 5; ++v) kv[v] = kv[v] - sh * (a.q[opt + v * N] - a.sp_qref[opt + v * N]);
+          }
+        }
+      }
       if (a.stage == 0) {
 #pragma unroll
         for (int v = 0; v < 5; ++v) a.rhs[pt + v * N] = kv[v];
@@ -647,16 +702,31 @@ bool fused_supported(const cruna_ctx *c) {
   return true;
 }
 
+static FusedArgs flow_args(const cruna_ctx *c) {
+  FusedArgs a;
+  a.g = c->g;
+  for (int d = 0; d < 3; ++d) a.op[d] = to_dir(c->dop[d], c->dx[d], c->cfg.heat_flux_dx != 0);
+  a.WoR = c->cfg.W / c->cfg.R;
+  a.mu0 = c->cfg.mu0;
+  a.T0 = c->cfg.T0;
+  a.gamma = c->cfg.gamma;
+  a.cp_over_pr = c->cfg.gamma * (c->cfg.R / c->cfg.W) / (c->cfg.gamma - 1.0) / c->cfg.Pr;
+  return a;
+}
+
+static void ensure_intermediates(cruna_ctx *c, bool fp32) {
+  if (c->fz) return;
+  void *p = nullptr;
+  CRUNA_CUDA_CHECK(cudaMalloc(&p, (size_t)NG * c->g.N * (fp32 ? sizeof(float) : sizeof(double))));
+  c->allocations.push_back(p);
+  c->fz = static_cast<double *>(p);
+}
+
 void rhs_direct_fused(cruna_ctx *c, const double *q_in, double *rhs, int stage, const double *q0, double *acc,
                       double *qnext, double dt) {
   const bool fp32 = c->cfg.precision == CRUNA_FP32_STENCIL;
   const long long N = c->g.N;
-  if (!c->fz) {
-    void *p = nullptr;
-    CRUNA_CUDA_CHECK(cudaMalloc(&p, (size_t)NG * N * (fp32 ? sizeof(float) : sizeof(double))));
-    c->allocations.push_back(p);
-    c->fz = static_cast<double *>(p);
-  }
+  ensure_intermediates(c, fp32);
   const double *q = q_in;
   if (c->has_q_bc) {                                               // ns_rho_rhou_p.f90:89-92
     copy_state(c, c->st[4], q_in, 5);
@@ -674,14 +744,7 @@ void rhs_direct_fused(cruna_ctx *c, const double *q_in, double *rhs, int stage, 
     c->T_ref = c->cfg.W / c->cfg.R * h[0] / h[1];
     c->refs_set = true;
   }
-  FusedArgs a;
-  a.g = c->g;
-  for (int d = 0; d < 3; ++d) a.op[d] = to_dir(c->dop[d], c->dx[d], c->cfg.heat_flux_dx != 0);
-  a.WoR = c->cfg.W / c->cfg.R;
-  a.mu0 = c->cfg.mu0;
-  a.T0 = c->cfg.T0;
-  a.gamma = c->cfg.gamma;
-  a.cp_over_pr = c->cfg.gamma * (c->cfg.R / c->cfg.W) / (c->cfg.gamma - 1.0) / c->cfg.Pr;
+  FusedArgs a = flow_args(c);
   a.p_ref = fp32 ? c->p_ref : 0.0;
   a.T_ref = fp32 ? c->T_ref : 0.0;
   a.q = q;
@@ -713,6 +776,81 @@ void rhs_direct_fused(cruna_ctx *c, const double *q_in, double *rhs, int stage, 
   if (stage == 0 || split) {
     if (c->has_rhs_bc) bc_rhs(c, rhs, q);                          // :218
     if (split) rk_stage(c, stage, dt, rhs, q0, acc, qnext);
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// compact schemes along y between explicit o8 ones along x and z: the z-marching passes for x and z, the
+// line engine's passes for y (dir_passes.cu).  684 bytes a point and RK stage (y flux pass 112, pass G 232, y
+// viscous pass 64, pass D 276) against 1040 with every direction on the line engine.
+// ------------------------------------------------------------------------------------------------
+bool march_y_supported(const cruna_ctx *c) {
+  for (int d : {0, 2}) {
+    const LineOp &op = c->dop[d];
+    if (op.kind != OP_STENCIL || op.solve || !op.periodic || op.r != 4) return false;
+  }
+  return c->dir_ok && c->dop[1].kind == OP_STENCIL && c->dop[1].solve;
+}
+
+void rhs_direct_march_y(cruna_ctx *c, const double *q_in, double *rhs, double *qbc, int bc_mask, int stage,
+                        const double *q0, double *acc, double *qnext, double dt) {
+  using Tv = double;
+  const long long N = c->g.N;
+  ensure_intermediates(c, false);
+  const double *q = q_in;
+  if (c->has_q_bc && (bc_mask & 1)) {                              // ns_rho_rhou_p.f90:89-92
+    copy_state(c, qbc, q_in, 5);
+    bc_q(c, qbc, 0);
+    q = qbc;
+  }
+  double *yr = c->tmp + (long long)F_M1 * N;
+  dir_flux(c, 1, q, c->tmp, yr, true);
+  const bool bcs = c->has_rhs_bc && (bc_mask & 2);
+  const bool split = bcs && !only_sponge(c);                       // other RHS boundary types act on the finished RHS
+  FusedArgs a = flow_args(c);
+  a.p_ref = a.T_ref = 0.0;
+  a.q = q;
+  a.gbuf = c->fz;
+  a.force = c->force;
+  a.yt = c->tmp;
+  a.yr = yr;
+  if (bcs && !split) {
+    a.sp_qref = c->qref;
+    a.sponge = c->sponge;
+  }
+  a.dt = dt;
+  a.q0 = q0;
+  a.acc = acc;
+  a.qnext = qnext;
+  a.stage = split ? 0 : stage;
+  a.rhs = a.stage == 0 ? rhs : nullptr;
+  constexpr int R = 4;
+  constexpr size_t sg = sizeof(Tv) * (6 * (TX + 2 * R) * TY + ring_slots(R) * 6 * TX * TY);
+  constexpr size_t sd = sizeof(Tv) * (4 * (TX + 2 * R) * TY + ring_slots(R) * 4 * TX * TY);
+  auto *kg = k_pass_g<Tv, R, true, false, true>;
+  auto *kd = k_pass_d<Tv, R, true, true>;
+  CRUNA_CUDA_CHECK(cudaFuncSetAttribute(kg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sg));
+  CRUNA_CUDA_CHECK(cudaFuncSetAttribute(kd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sd));
+  static const int res_g = resident_blocks(kg, TX * TY, sg), res_d = resident_blocks(kd, TX * TY, sd);
+  const int bx = (c->g.n1 + TX - 1) / TX, by = (c->g.n2 + TY - 1) / TY;
+  int nz = 1;
+  {
+    a.kc = z_chunk_balanced(c->g.n3, bx * by, res_g, device_sms(), R, nz);
+    ProfScope ps(c, "pass_g_xz");
+    kg<<<dim3(bx, by, nz), dim3(TX, TY), sg, c->stream>>>(a);
+    CRUNA_LAUNCH_CHECK(c);
+  }
+  double *G = c->fz;                                               // tau_12, tau_22, tau_23, lambda T_y; onto c2..c5
+  dir_viscous(c, 1, G + 6 * N, G + 8 * N, G + 9 * N, G + 12 * N, G);
+  {
+    a.kc = z_chunk_balanced(c->g.n3, bx * by, res_d, device_sms(), R, nz);
+    ProfScope ps(c, "pass_d_xz");
+    kd<<<dim3(bx, by, nz), dim3(TX, TY), sd, c->stream>>>(a);
+    CRUNA_LAUNCH_CHECK(c);
+  }
+  if (split) {
+    bc_rhs(c, rhs, q);                                             // :218
+    if (stage) rk_stage(c, stage, dt, rhs, q0, acc, qnext);
   }
 }
 

@@ -34,6 +34,7 @@ struct AdjArgs {
   const double *q0;
   double *acc;
   double *qnext;
+  const double *yr;    // YX: the y direction's terms of the five equations, from the line engine
 };
 
 // per-direction contribution in the reference's order (ns_rho_rhou_p.f90:317-370 / 386-440 / 456-509)
@@ -75,11 +76,13 @@ __device__ __forceinline__ void adj_dir(int d, double u1, double u2, double u3, 
 // plane fields: 0..4 qs1..qs5, 5 p - p_ref, 6 u, 7 v ; column fields: 0..4 qs1..qs5, 5 p - p_ref, 6 w.
 // T is the type of the shared-memory fields and of the derivatives (double, or float for the
 // FP32-stencil precision); the assembly and the RK update stay in double.
-template <typename T, int R, bool PER>
+// YX: without the y derivatives (compact schemes along y), starting from a.yr: no y halos, no v in the plane.
+template <typename T, int R, bool PER, bool YX = false>
 __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(const __grid_constant__ AdjArgs a) {
-  constexpr int PW = TX + 2 * R, PH = TY + 2 * R, PS = PW * PH;
+  constexpr int RY = YX ? 0 : R;
+  constexpr int PW = TX + 2 * R, PH = TY + 2 * RY, PS = PW * PH;
   constexpr int NS = ring_slots(R);
-  constexpr int NPF = 8, NRF = 7, RS = TX * TY;
+  constexpr int NPF = YX ? 7 : 8, NRF = 7, RS = TX * TY;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *plane = reinterpret_cast<T *>(smem_raw);          // [NPF][PH][PW]
   T *ring = plane + NPF * PS;                          // [NS][NRF][TY*TX]
@@ -96,7 +99,7 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
   const int colpt = gi + n1 * gj;
   const double *S0 = a.qs, *S1 = a.qs + N, *S2 = a.qs + 2 * N, *S3 = a.qs + 3 * N, *S4 = a.qs + 4 * N;
   const double *Q0 = a.q, *Q1 = a.q + N, *Q2 = a.q + 2 * N, *Q3 = a.q + 3 * N, *Q4 = a.q + 4 * N;
-  HaloSet<R> hs;
+  HaloSet<R, RY> hs;
   hs.init(ox, oy, i0, j0, tid, n1);
 
   auto put_ring = [&](int kk, const double *v8) {
@@ -135,7 +138,7 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
     }
   };
   prefetch(k0 + R, k0);
-  constexpr int NHT = HaloSet<R>::PER_THREAD;
+  constexpr int NHT = HaloSet<R, RY>::PER_THREAD;
   double hv[NHT][9];      // qs1..qs5, rho, rho*u, rho*v, p of the halo cells, one plane ahead
   auto halo_fetch = [&](int kk) {
     const long long kofs = (long long)n12 * kk;
@@ -144,7 +147,8 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
       if (hs.goff[h] < 0) continue;
       const long long pt = hs.goff[h] + kofs;
       hv[h][0] = S0[pt]; hv[h][1] = S1[pt]; hv[h][2] = S2[pt]; hv[h][3] = S3[pt]; hv[h][4] = S4[pt];
-      hv[h][5] = Q0[pt]; hv[h][6] = Q1[pt]; hv[h][7] = Q2[pt]; hv[h][8] = Q4[pt];
+      hv[h][5] = Q0[pt]; hv[h][6] = Q1[pt]; hv[h][8] = Q4[pt];
+      if constexpr (!YX) hv[h][7] = Q2[pt];
     }
   };
   halo_fetch(k0);
@@ -155,18 +159,22 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
     const double ir = 1.0 / rho_c;                            // ns_rho_rhou_p.f90:294
     const double u1 = pc[1] * ir, u2 = pc[2] * ir;
     {
-      T *c = plane + (ty + R) * PW + (tx + R);
+      T *c = plane + (ty + RY) * PW + (tx + R);
       const T *rp = ring + slot * NRF * RS + tid;
 #pragma unroll
       for (int f = 0; f < 6; ++f) c[f * PS] = rp[f * RS];
       c[6 * PS] = T(u1);
-      c[7 * PS] = T(u2);
+      if constexpr (!YX) c[7 * PS] = T(u2);
     }
     const long long kofs = (long long)n12 * k;
     // epilogue inputs of this plane, issued before the barrier so their latency overlaps the stencils
     const long long opt = (i0 + tx) + (long long)n1 * (j0 + ty) + kofs;
-    double e_src[5] = {0, 0, 0, 0, 0}, e_q0[5] = {0, 0, 0, 0, 0}, e_acc[5] = {0, 0, 0, 0, 0};
+    double e_y[5] = {0, 0, 0, 0, 0}, e_src[5] = {0, 0, 0, 0, 0}, e_q0[5] = {0, 0, 0, 0, 0}, e_acc[5] = {0, 0, 0, 0, 0};
     if (inside) {
+      if constexpr (YX) {
+#pragma unroll
+        for (int v = 0; v < 5; ++v) e_y[v] = a.yr[opt + v * N];
+      }
       if (a.src) {
 #pragma unroll
         for (int v = 0; v < 5; ++v) e_src[v] = a.src[opt + v * N];
@@ -189,14 +197,14 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
       const double hir = 1.0 / hv[h][5];
       c[5 * PS] = T(hv[h][8] - a.p_ref);
       c[6 * PS] = T(hv[h][6] * hir);
-      c[7 * PS] = T(hv[h][7] * hir);
+      if constexpr (!YX) c[7 * PS] = T(hv[h][7] * hir);
     }
     prefetch(k + R + 1, k + 1);
     if (k + 1 < k1) halo_fetch(k + 1);
     __syncthreads();
     if (inside) {
       const int i = i0 + tx, j = j0 + ty;
-      const T *c = plane + (ty + R) * PW + (tx + R);
+      const T *c = plane + (ty + RY) * PW + (tx + R);
       int so[NS];
 #pragma unroll
       for (int m = -R; m <= R; ++m) so[m + R] = ((slot + m + NS) % NS) * NRF * RS + tid;
@@ -204,7 +212,7 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
       const double gm1 = a.gamma - 1.0;
       const double u3 = ring[so[R] + 6 * RS];
       const double gpr = a.gamma * p_c / (rho_c * gm1);         // :293
-      double r1 = 0.0, r2 = 0.0, r3 = 0.0, r4 = 0.0, r5 = 0.0;  // :296
+      double r1 = e_y[0], r2 = e_y[1], r3 = e_y[2], r4 = e_y[3], r5 = e_y[4];  // :296
       {
         const double s = ox.scale;
         const double A = D1<T, R, PER>(ox, c, 1, i) * s, B = D1<T, R, PER>(ox, c + PS, 1, i) * s,
@@ -214,7 +222,7 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
         const double P = D1<T, R, PER>(ox, c + 5 * PS, 1, i) * s;
         adj_dir(0, u1, u2, u3, gpr, ir, qs5, a.gamma, A, B, Cc, D, E, Sx, P, r1, r2, r3, r4, r5);
       }
-      {
+      if constexpr (!YX) {
         const double s = oy.scale;
         const double A = D1<T, R, PER>(oy, c, PW, j) * s, B = D1<T, R, PER>(oy, c + PS, PW, j) * s,
                      Cc = D1<T, R, PER>(oy, c + 2 * PS, PW, j) * s, D = D1<T, R, PER>(oy, c + 3 * PS, PW, j) * s,
@@ -753,6 +761,53 @@ void rhs_adjoint_fused(cruna_ctx *c, const double *qs_in, const double *q, const
   if (stage == 0 || split) {
     if (c->has_rhs_bc) bc_rhss(c, rhs, qs, nullptr);                // :518 (without q)
     if (split) rk_stage(c, stage, dt, rhs, qs0, acc, qnext);
+  }
+}
+
+// adjoint RHS or RK stage with a compact scheme along y (march_y_supported): the y terms from the line
+// engine, x and z and the stage update in the z-marching pass.  380 bytes a point and stage against 560.
+void rhs_adjoint_march_y(cruna_ctx *c, const double *qs_in, const double *q, const double *g, double *rhs, double *qsbc,
+                         int stage, const double *qs0, double *acc, double *qnext, double dt) {
+  const double *qs = qs_in;
+  if (c->has_q_bc) {                                               // ns_rho_rhou_p.f90:287-290
+    copy_state(c, qsbc, qs_in, 5);
+    bc_qs(c, qsbc, q, 0);
+    qs = qsbc;
+  }
+  dir_adjoint(c, 1, qs, q, c->tmp, true);
+  bool walls = false;                                              // :518 without q: only the walls act
+  for (const BCRow &b : c->bc) walls = walls || b.type == 100;
+  AdjArgs a;
+  a.g = c->g;
+  a.p_ref = 0.0;
+  for (int d = 0; d < 3; ++d) a.op[d] = to_dir(c->dop[d], c->dx[d], true);
+  a.gamma = c->cfg.gamma;
+  a.qs = qs;
+  a.q = q;
+  a.src = g;
+  a.dt = dt;
+  a.q0 = qs0;
+  a.acc = acc;
+  a.qnext = qnext;
+  a.yr = c->tmp;
+  a.stage = walls ? 0 : stage;
+  a.rhs = a.stage == 0 ? rhs : nullptr;
+  constexpr int R = 4;
+  constexpr size_t sm = sizeof(double) * (7 * (TX + 2 * R) * TY + ring_slots(R) * 7 * TX * TY);
+  auto *k = k_adj_pass<double, R, true, true>;
+  CRUNA_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  static const int res = resident_blocks(k, TX * TY, sm);
+  const int bx = (c->g.n1 + TX - 1) / TX, by = (c->g.n2 + TY - 1) / TY;
+  int nz = 1;
+  a.kc = z_chunk_balanced(c->g.n3, bx * by, res, device_sms(), R, nz);
+  {
+    ProfScope ps(c, "adj_pass_xz");
+    k<<<dim3(bx, by, nz), dim3(TX, TY), sm, c->stream>>>(a);
+    CRUNA_LAUNCH_CHECK(c);
+  }
+  if (walls) {
+    bc_rhss(c, rhs, qs, nullptr);
+    if (stage) rk_stage(c, stage, dt, rhs, qs0, acc, qnext);
   }
 }
 

@@ -51,6 +51,10 @@ struct FusedArgs {
   double cl_delta = 0.0;
   int cl_norm = 0;
   int *cl_err = nullptr;
+  // y derivatives from the line engine (YX instantiations): gradients u_y, v_y, w_y, T_y in the generic
+  // workspace's slots, the five convective accumulators, and the type-400 sponge of the RHS (null: none)
+  const double *yt = nullptr, *yr = nullptr, *sp_qref = nullptr;
+  SpongeDev sponge;
 };
 
 __host__ __device__ constexpr int ring_slots(int R) { return 2 * R + 1; }
@@ -297,7 +301,7 @@ __device__ __forceinline__ T Dz2(const DirOpF &op, const T *a, const T *b, int k
   else return dsz2<T, R>(op, a, b, k);
 }
 
-// halo strip cell h (no corners) of a TX x TY tile with R-wide halos -> local (lx, ly)
+// halo strip cell h (no corners) of a TX x TY tile with R-wide halos (the x strips come first) -> local (lx, ly)
 template <int R>
 __device__ __forceinline__ void halo_cell(int h, int &lx, int &ly) {
   if (h < 2 * R * TY) {
@@ -312,10 +316,11 @@ __device__ __forceinline__ void halo_cell(int h, int &lx, int &ly) {
   }
 }
 
-// per-thread halo cells: smem cell offset and in-plane global offset (-1: outside an open line)
-template <int R>
+// per-thread halo cells: smem cell offset and in-plane global offset (-1: outside an open line); RY = 0:
+// x strips only, on a tile without y halos
+template <int R, int RY = R>
 struct HaloSet {
-  static constexpr int NH = 2 * R * (TX + TY);
+  static constexpr int NH = 2 * R * TY + 2 * RY * TX;
   static constexpr int PER_THREAD = (NH + TX * TY - 1) / (TX * TY);
   int cell[PER_THREAD];
   int goff[PER_THREAD];
@@ -330,7 +335,7 @@ struct HaloSet {
         int lx, ly;
         halo_cell<R>(h, lx, ly);
         const int hi = gidx(ox, i0 + lx), hj = gidx(oy, j0 + ly);
-        cell[c] = (ly + R) * PW + (lx + R);
+        cell[c] = (ly + RY) * PW + (lx + R);
         if (hi >= 0 && hj >= 0) goff[c] = hi + n1 * hj;
       }
     }

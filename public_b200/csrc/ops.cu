@@ -7,6 +7,7 @@
 
 #include "bc_point.cuh"
 #include "cruna_internal.cuh"
+#include "lines.cuh"
 #include "ops_common.cuh"
 
 namespace cruna {
@@ -71,10 +72,9 @@ __global__ void k_line_solve(LineOp op, Grid g, int dir, double *__restrict__ da
 }
 
 // ------------------------------------------------------------------------------------------------
-// fast line operators: the same arithmetic as k_line_stencil / k_line_solve (identical expressions in
-// identical order, so identical results), with the interior radius a compile-time constant, no
-// integer division per tap, and for compact operators along y and z the explicit part and the
-// dgttrs sweeps fused in one pass over each line
+// fast line operators: the same arithmetic as k_line_stencil (identical expressions in identical order,
+// so identical results), with the interior radius a compile-time constant and no integer division per tap;
+// compact operators take the explicit part and the solve in one pass over each line
 // ------------------------------------------------------------------------------------------------
 
 // interior explicit part from values v(m) = f(i + m), m = -R..R, in explicit_part's order
@@ -165,172 +165,73 @@ __global__ void __launch_bounds__(128) k_line_stencil_r(LineOp op, Grid g, const
   }
 }
 
-// Compact operators along y or z: one thread per line, consecutive threads on consecutive x (every
-// load and store coalesced).  The operator's factors sit in shared memory (the same for every line).
-// EXPL: the explicit part comes from a sliding window of f over the interior (one new load per point;
-// the closure rows of open lines use explicit_part) and dgttrs's forward sweep runs on the fly;
-// otherwise the line of `out` is solved in place.  Then the backward sweep and the cyclic correction
-// over the stored forward values.  Every sweep reads its line CH points at a time and issues the next
-// chunk's loads before it works through the current one, so two chunks' loads are in flight.
-constexpr int kCompactMaxN = 1024;  // factors in shared memory: 44 bytes per line point
-
-template <int R, bool ANTI, bool EXPL, bool NOPIV>
-__global__ void __launch_bounds__(64) k_line_compact_yz(LineOp op, Grid g, int dir,
-                                                        const double *__restrict__ f1,
-                                                        const double *__restrict__ f2, double *out,
-                                                        double scale, double sign, int nfields) {
-  constexpr int CH = 8;
-  constexpr int W = 2 * R + 1;
-  extern __shared__ double cs[];
+// Compact operators (explicit part, tridiagonal solve, cyclic correction) on the line engine, one field per
+// blockIdx.y; R = 0 solves the input itself.  Every load of a block precedes its first barrier and its stores
+// follow one, and a block owns whole lines, so out may be the input.  X: lines along x, staged through
+// shared memory with an odd row pitch (lanes on neighbouring lines then hit different banks).
+template <int R, bool ANTI, bool X>
+__global__ void __launch_bounds__(kLineThreads, 3) k_lines(const __grid_constant__ LineOp op, Grid g, int dir,
+                                                  const __grid_constant__ FieldSet fs, double scale, int G, int C) {
+  extern __shared__ double line_sm[];
+  const LineBlock b = line_block<1>(op, line_sm, G, C);
   const int n = op.n;
-  double *s_dl = cs, *s_du = cs + n, *s_du2 = cs + 2 * n, *s_inv = cs + 3 * n, *s_fb = cs + 4 * n;
-  int *s_piv = reinterpret_cast<int *>(cs + 5 * n);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    s_dl[i] = i < n - 1 ? op.dl[i] : 0.0;
-    s_du[i] = i < n - 1 ? op.du[i] : 0.0;
-    s_du2[i] = i < n - 2 ? op.du2[i] : 0.0;
-    s_inv[i] = op.inv_d[i];
-    s_fb[i] = op.cyclic ? op.fbnorm[i] : 0.0;
-    s_piv[i] = NOPIV ? i + 1 : op.ipiv[i];
-  }
-  __syncthreads();
-  const long long n12 = (long long)g.n1 * g.n2;
-  const long long nlines = g.N / n;
-  const long long total = nlines * nfields;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const long long fld = t / nlines, l = t - fld * nlines;
-    long long base, s;
-    if (dir == 1) { const long long i = l % g.n1, k = l / g.n1; base = i + k * n12; s = g.n1; }
-    else { base = l; s = n12; }
-    double *o = out + fld * g.N + base;
-    double *po = o;  // o[(i - 1) * s] for the forward step at i
-    double cur = 0.0;
-    // dgttrs forward sweep (L with LAPACK's row interchanges) on the pair (i - 1, i); v = b[i]
-    auto fwd = [&](int i, double v) {
-      if (i == 0) {
-        cur = v;
-        return;
-      }
-      if (NOPIV || s_piv[i - 1] == i) {
-        *po = cur;
-        cur = v - s_dl[i - 1] * cur;
-      } else {
-        *po = v;
-        cur = cur - s_dl[i - 1] * v;
-      }
-      po += s;
-    };
-    if (EXPL) {
-      const double *a = f1 + fld * g.N + base;
-      const double *b = f2 ? f2 + fld * g.N + base : nullptr;
-      const int ib = op.periodic ? 0 : op.nb, ie = op.periodic ? n : n - op.nb;
-      for (int i = 0; i < ib; ++i)
-        fwd(i, point_epilogue(op, explicit_part(op, a, b, 0, s, i), ldv(a, b, i * s), scale, sign));
-      auto wrap = [&](int idx) { return op.periodic ? (idx < 0 ? idx + n : (idx >= n ? idx - n : idx)) : idx; };
-      double w[W];  // w[R + m] = f(i + m)
-#pragma unroll
-      for (int m = 0; m < W; ++m) w[m] = ldv(a, b, wrap(ib + m - R) * s);
-      auto step = [&](int i, double next) {  // position i from the window, then slide it by one
-        const double v = interior_part<R, ANTI>(op, [&](int m) { return w[R + m]; });
-        fwd(i, point_epilogue(op, v, w[R], scale, sign));
-#pragma unroll
-        for (int m = 0; m < W - 1; ++m) w[m] = w[m + 1];
-        w[W - 1] = next;
-      };
-      // chunk at i0 needs f(i0 + u + 1 + R), u < CH, while i0 + u + 1 < ie
-      int i0 = ib;
-      double nx[CH];
-      if (i0 + CH <= ie) {
-#pragma unroll
-        for (int u = 0; u < CH; ++u) nx[u] = (i0 + u + 1 < ie) ? ldv(a, b, wrap(i0 + u + 1 + R) * s) : 0.0;
-      }
-      for (; i0 + CH <= ie; i0 += CH) {
-        double cb[CH];
-#pragma unroll
-        for (int u = 0; u < CH; ++u) cb[u] = nx[u];
-        if (i0 + 2 * CH <= ie) {
-#pragma unroll
-          for (int u = 0; u < CH; ++u)
-            nx[u] = (i0 + CH + u + 1 < ie) ? ldv(a, b, wrap(i0 + CH + u + 1 + R) * s) : 0.0;
+  const int nlines = (int)(g.N / n), l0 = blockIdx.x * G, line = l0 + b.g;
+  const double *f1 = fs.f1[blockIdx.y], *f2 = fs.f2[blockIdx.y];
+  double *out = fs.out[blockIdx.y];
+  double v[1][kLineL];
+  double w[kLineL + 2 * R];
+  if constexpr (X) {
+    double *tile = b.ends + 2 * G;
+    const int pitch = n | 1;
+    const int base = l0 * n, count = min(G, nlines - l0) * n;
+    auto each = [&](auto fn) {  // the block's points in memory order and their places in the tile
+      int l = threadIdx.x / n, x = threadIdx.x - l * n;
+      for (int p = threadIdx.x; p < count; p += blockDim.x) {
+        fn(base + p, l * pitch + x);
+        x += blockDim.x;
+        while (x >= n) {
+          x -= n;
+          ++l;
         }
-#pragma unroll
-        for (int u = 0; u < CH; ++u) step(i0 + u, cb[u]);
       }
-      for (; i0 < ie; ++i0) step(i0, (i0 + 1 < ie) ? ldv(a, b, wrap(i0 + 1 + R) * s) : 0.0);
-      for (int i = ie; i < n; ++i)
-        fwd(i, point_epilogue(op, explicit_part(op, a, b, 0, s, i), ldv(a, b, i * s), scale, sign));
-    } else {
-      cur = o[0];
-      const double *pl = o + s;  // o[i0 * s]
-      int i0 = 1;
-      double nx[CH];
-      if (i0 + CH <= n) {
-#pragma unroll
-        for (int u = 0; u < CH; ++u) nx[u] = pl[(long long)u * s];
-      }
-      for (; i0 + CH <= n; i0 += CH) {
-        double cb[CH];
-#pragma unroll
-        for (int u = 0; u < CH; ++u) cb[u] = nx[u];
-        pl += CH * s;
-        if (i0 + 2 * CH <= n) {
-#pragma unroll
-          for (int u = 0; u < CH; ++u) nx[u] = pl[(long long)u * s];
-        }
-#pragma unroll
-        for (int u = 0; u < CH; ++u) fwd(i0 + u, cb[u]);
-      }
-      for (; i0 < n; ++i0, pl += s) fwd(i0, *pl);
-    }
-    // backward sweep with U (diagonal inverted, du, du2); po now points at o[(n - 1) * s]
-    double x2 = cur * s_inv[n - 1];
-    *po = x2;
-    const double xlast = x2;
-    double x1 = (po[-s] - s_du[n - 2] * x2) * s_inv[n - 2];  // n > 2R + 2 >= 4
-    po -= s;
-    *po = x1;
-    auto back = [&](int i, double bi) {
-      const double x0 = (bi - s_du[i] * x1 - s_du2[i] * x2) * s_inv[i];
-      po -= s;
-      *po = x0;
-      x2 = x1;
-      x1 = x0;
     };
-    int i0 = n - 3;  // chunk at i0 reads positions i0 - u = po[-(u + 1) s]
-    double nb[CH];
-    if (i0 >= CH - 1) {
+    each([&](int p, int at) { tile[at] = f2 ? f1[p] * f2[p] : f1[p]; });
+    __syncthreads();
+    const double *row = tile + b.g * pitch;
+    auto f = [&](int i) { return row[i]; };
+    line_window<R>(op, b.i0, f, w);
+    line_explicit<R, ANTI>(op, b.i0, w, f, v[0]);
+    if (ANTI) {
 #pragma unroll
-      for (int u = 0; u < CH; ++u) nb[u] = po[-(long long)(u + 1) * s];
+      for (int k = 0; k < kLineL; ++k) v[0][k] = v[0][k] * scale;
     }
-    for (; i0 >= CH - 1; i0 -= CH) {
-      double cb[CH];
+    line_solve<1>(op, b, v);  // its barriers follow every read of the tile
 #pragma unroll
-      for (int u = 0; u < CH; ++u) cb[u] = nb[u];
-      if (i0 - CH >= CH - 1) {
+    for (int k = 0; k < kLineL; ++k)
+      if (b.i0 + k < n) tile[b.g * pitch + b.i0 + k] = v[0][k];
+    __syncthreads();
+    each([&](int p, int at) { out[p] = tile[at]; });
+  } else {
+    int base = 0, s = 0;
+    line_base(g, dir, min(line, nlines - 1), base, s);
+    const double *p1 = f1 + base, *p2 = f2 ? f2 + base : nullptr;
+    auto f = [&](int i) { return p2 ? p1[i * s] * p2[i * s] : p1[i * s]; };
+    line_window<R>(op, b.i0, f, w);
+    line_explicit<R, ANTI>(op, b.i0, w, f, v[0]);
+    if (ANTI) {
 #pragma unroll
-        for (int u = 0; u < CH; ++u) nb[u] = po[-(long long)(CH + u + 1) * s];
-      }
-#pragma unroll
-      for (int u = 0; u < CH; ++u) back(i0 - u, cb[u]);
+      for (int k = 0; k < kLineL; ++k) v[0][k] = v[0][k] * scale;
     }
-    for (; i0 >= 0; --i0) back(i0, po[-s]);
-    if (op.cyclic) {  // Sherman-Morrison: x1 is the solution's first value, xlast its last
-      const double corr = x1 + op.fbrat * xlast;
-      for (int j0 = 0; j0 < n; j0 += CH) {
-        double bv[CH];
+    __syncthreads();  // the row table
+    line_solve<1>(op, b, v);
+    if (line < nlines) {
+      double *o = out + base;
 #pragma unroll
-        for (int u = 0; u < CH; ++u) bv[u] = (j0 + u < n) ? o[(long long)(j0 + u) * s] : 0.0;
-#pragma unroll
-        for (int u = 0; u < CH; ++u)
-          if (j0 + u < n) o[(long long)(j0 + u) * s] = bv[u] - s_fb[j0 + u] * corr;
-      }
+      for (int k = 0; k < kLineL; ++k)
+        if (b.i0 + k < n) o[(b.i0 + k) * s] = v[0][k];
     }
   }
 }
-
-static size_t compact_smem(const LineOp &op) { return (size_t)op.n * (5 * sizeof(double) + sizeof(int)); }
-
 
 // the fast kernels handle interior radii 1..6 on lines longer than 2R + 2 (every periodic wrap then
 // stays within one period) whose open ends have at least R closure rows and an interior between them
@@ -371,26 +272,21 @@ static void launch_stencil_r(cruna_ctx *c, const LineOp &op, int dir, const Fiel
   }
 }
 
-template <bool ANTI>
-static void launch_compact_r(cruna_ctx *c, const LineOp &op, int dir, const double *f1, const double *f2,
-                             double *out, double scale, double sign, int nfields) {
-  const long long lines = (c->g.N / op.n) * nfields;
-  const int blocks = nblocks(lines, 64);  // one line per thread: small blocks spread few lines over all SMs
-  const size_t sm = compact_smem(op);
-  switch (op.r) {
-#define CRUNA_COMPACT_CASE(RR)                                                                          \
-  case RR:                                                                                              \
-    if (op.nopiv)                                                                                       \
-      k_line_compact_yz<RR, ANTI, true, true><<<blocks, 64, sm, c->stream>>>(op, c->g, dir, f1, f2, out, scale, \
-                                                                             sign, nfields);            \
-    else                                                                                                \
-      k_line_compact_yz<RR, ANTI, true, false><<<blocks, 64, sm, c->stream>>>(op, c->g, dir, f1, f2, out, scale, \
-                                                                              sign, nfields);           \
-    break;
-    CRUNA_COMPACT_CASE(1) CRUNA_COMPACT_CASE(2) CRUNA_COMPACT_CASE(3)
-    CRUNA_COMPACT_CASE(4) CRUNA_COMPACT_CASE(5) CRUNA_COMPACT_CASE(6)
-#undef CRUNA_COMPACT_CASE
-  }
+template <int R, bool ANTI, bool X>
+static void launch_lines_r(cruna_ctx *c, const LineOp &op, int dir, const FieldSet &fs, double scale) {
+  const int C = line_chunks(op.n), G = line_group(C);
+  const long long lines = c->g.N / op.n;
+  const size_t sm = sizeof(double) * (line_smem_doubles(C, G, 1) + (X ? (size_t)G * (op.n | 1) : 0));
+  if (sm > 48 * 1024)
+    CRUNA_CUDA_CHECK(cudaFuncSetAttribute(k_lines<R, ANTI, X>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  k_lines<R, ANTI, X><<<dim3((unsigned)((lines + G - 1) / G), fs.n), C * G, sm, c->stream>>>(op, c->g, dir, fs, scale, G, C);
+}
+
+template <int R, bool ANTI>
+static void launch_lines(cruna_ctx *c, const LineOp &op, int dir, const FieldSet &fs, double scale) {
+  if (dir == 0) launch_lines_r<R, ANTI, true>(c, op, dir, fs, scale);
+  else launch_lines_r<R, ANTI, false>(c, op, dir, fs, scale);
+  CRUNA_LAUNCH_CHECK(c);
 }
 
 // contiguous fields f1 + k N (f2 + k N), out + k N, k < nfields, as field sets of at most kMax
@@ -408,8 +304,10 @@ static const char *const kStencilNames[2][3] = {{"line_filter_x", "line_filter_y
                                                 {"line_diff_x", "line_diff_y", "line_diff_z"}};
 
 static bool stencil_fast(const cruna_ctx *c, const LineOp &op) { return fast_ok(op) && c->g.n2 <= 65535; }
-static bool compact_fast(const LineOp &op, int dir) {
-  return op.kind == OP_STENCIL && op.solve && dir > 0 && fast_ok(op) && op.n <= kCompactMaxN;
+// compact operators on the line engine: every scheme of the tables above (derivatives of radius 1 and 2, filters
+// of radius 1 to 5) up to kLineMaxN points a line
+static bool compact_fast(const cruna_ctx *c, const LineOp &op) {
+  return line_grid_ok(c->g) && op.kind == OP_STENCIL && op.solve && op.tab && op.r <= (op.antisym ? 2 : 5);
 }
 
 static void launch_stencil_set(cruna_ctx *c, const LineOp &op, int dir, const FieldSet &fs, double scale,
@@ -436,42 +334,44 @@ void launch_line_stencil(cruna_ctx *c, const LineOp &op, int dir, const double *
 void launch_line_solve(cruna_ctx *c, const LineOp &op, int dir, double *data, int nfields) {
   static const char *names[3] = {"line_solve_x", "line_solve_y", "line_solve_z"};
   ProfScope ps(c, names[dir]);
-  const long long lines = (c->g.N / op.n) * nfields;
-  if (dir > 0 && op.n >= 4 && op.n <= kCompactMaxN) {
-    if (op.nopiv)
-      k_line_compact_yz<1, false, false, true><<<nblocks(lines, 64), 64, compact_smem(op), c->stream>>>(
-          op, c->g, dir, nullptr, nullptr, data, 1.0, 1.0, nfields);
-    else
-      k_line_compact_yz<1, false, false, false><<<nblocks(lines, 64), 64, compact_smem(op), c->stream>>>(
-          op, c->g, dir, nullptr, nullptr, data, 1.0, 1.0, nfields);
-    CRUNA_LAUNCH_CHECK(c);
+  if (op.tab && line_grid_ok(c->g)) {
+    for_sets(c, data, nullptr, data, nfields, [&](const FieldSet &fs) { launch_lines<0, false>(c, op, dir, fs, 1.0); });
     return;
   }
+  const long long lines = (c->g.N / op.n) * nfields;
   k_line_solve<<<nblocks(lines, 128), 128, 0, c->stream>>>(op, c->g, dir, data, nfields);
   CRUNA_LAUNCH_CHECK(c);
 }
 
-// explicit part and compact solve of op along y or z in one pass (compact_fast(op, dir)) on nfields
-// contiguous fields
-static void launch_line_compact(cruna_ctx *c, const LineOp &op, int dir, const double *f1, const double *f2,
-                                double *out, double scale, int nfields) {
-  static const char *names[2][3] = {{"", "compact_filter_y", "compact_filter_z"},
-                                    {"", "compact_diff_y", "compact_diff_z"}};
+// explicit part and compact solve of op (compact_fast(op)) of every field of a set in one launch
+static void launch_compact_set(cruna_ctx *c, const LineOp &op, int dir, const FieldSet &fs, double scale) {
+  static const char *names[2][3] = {{"compact_filter_x", "compact_filter_y", "compact_filter_z"},
+                                    {"compact_diff_x", "compact_diff_y", "compact_diff_z"}};
   ProfScope ps(c, names[op.antisym ? 1 : 0][dir]);
-  if (op.antisym) launch_compact_r<true>(c, op, dir, f1, f2, out, scale, 1.0, nfields);
-  else launch_compact_r<false>(c, op, dir, f1, f2, out, scale, 1.0, nfields);
-  CRUNA_LAUNCH_CHECK(c);
+  if (op.antisym) {
+    if (op.r == 1) launch_lines<1, true>(c, op, dir, fs, scale);
+    else launch_lines<2, true>(c, op, dir, fs, scale);
+    return;
+  }
+  switch (op.r) {
+    case 1: launch_lines<1, false>(c, op, dir, fs, scale); break;
+    case 2: launch_lines<2, false>(c, op, dir, fs, scale); break;
+    case 3: launch_lines<3, false>(c, op, dir, fs, scale); break;
+    case 4: launch_lines<4, false>(c, op, dir, fs, scale); break;
+    default: launch_lines<5, false>(c, op, dir, fs, scale); break;
+  }
 }
 
-// Dx_d of each field of a set (f1, or f1*f2 when every f2 is given), all with the same spacing h:
-// explicit operators take one launch per set; compact ones (whose kernel keeps one line per thread in
-// flight, so more fields per launch do not shorten it) and the fallbacks one apply_diff per field
+// Dx_d of each field of a set (f1, or f1*f2 when every f2 is given), all with the same spacing h, in one
+// launch; the fallbacks take one apply_diff per field
 void apply_diff_set(cruna_ctx *c, int dir, const FieldSet &fs, double h) {
   const LineOp &op = c->dop[dir];
   const double scale = 1.0 / (h * op.div);
   bool uniform = true;
   for (int k = 1; k < fs.n; ++k) uniform = uniform && ((fs.f2[k] != nullptr) == (fs.f2[0] != nullptr));
-  if (uniform && !op.solve && stencil_fast(c, op)) {
+  if (compact_fast(c, op)) {
+    launch_compact_set(c, op, dir, fs, scale);
+  } else if (uniform && !op.solve && stencil_fast(c, op)) {
     launch_stencil_set(c, op, dir, fs, scale, 1.0);
   } else {
     for (int k = 0; k < fs.n; ++k) apply_diff(c, dir, fs.f1[k], fs.f2[k], fs.out[k], h, 1);
@@ -483,24 +383,25 @@ void apply_diff(cruna_ctx *c, int dir, const double *f1, const double *f2, doubl
                 int nfields) {
   const LineOp &op = c->dop[dir];
   const double scale = 1.0 / (h * op.div);
-  if (compact_fast(op, dir)) {
-    launch_line_compact(c, op, dir, f1, f2, out, scale, nfields);
+  if (compact_fast(c, op)) {
+    for_sets(c, f1, f2, out, nfields, [&](const FieldSet &fs) { launch_compact_set(c, op, dir, fs, scale); });
     return;
   }
   launch_line_stencil(c, op, dir, f1, f2, out, scale, nfields);
   if (op.kind == OP_STENCIL && op.solve) launch_line_solve(c, op, dir, out, nfields);
 }
 
-// filter_i_d in place: out-of-place stencil into scratch, solve, copy back
+// filter_i_d in place: compact filters on the line engine, which works in place; the others out of place
+// into scratch, solve, copy back
 void apply_filter(cruna_ctx *c, int dir, double *q, double *scratch, int nfields) {
   const LineOp &op = c->fop[dir];
   if (op.kind == OP_COPY) return;
-  if (compact_fast(op, dir)) {
-    launch_line_compact(c, op, dir, q, nullptr, scratch, 1.0, nfields);
-  } else {
-    launch_line_stencil(c, op, dir, q, nullptr, scratch, 1.0, nfields);
-    if (op.solve) launch_line_solve(c, op, dir, scratch, nfields);
+  if (compact_fast(c, op)) {
+    for_sets(c, q, nullptr, q, nfields, [&](const FieldSet &fs) { launch_compact_set(c, op, dir, fs, 1.0); });
+    return;
   }
+  launch_line_stencil(c, op, dir, q, nullptr, scratch, 1.0, nfields);
+  if (op.solve) launch_line_solve(c, op, dir, scratch, nfields);
   CRUNA_CUDA_CHECK(cudaMemcpyAsync(q, scratch, sizeof(double) * c->g.N * nfields,
                                    cudaMemcpyDeviceToDevice, c->stream));
 }
@@ -944,7 +845,29 @@ __global__ void k_assemble(long long N, const double *__restrict__ t, double *__
   }
 }
 
+void stage_direct_generic(cruna_ctx *c, const double *q, double *k, double *qbc, int stage, const double *q0,
+                          double *acc, double *qnext, double dt) {
+  if (c->march_y_ok) {
+    rhs_direct_march_y(c, q, k, qbc, 3, stage, q0, acc, qnext, dt);
+    return;
+  }
+  if (c->dir_ok) {
+    rhs_direct_dir(c, q, k, qbc, 3, stage, q0, acc, qnext, dt);
+    return;
+  }
+  rhs_direct_generic(c, q, k, qbc);
+  rk_stage(c, stage, dt, k, q0, acc, qnext);
+}
+
 void rhs_direct_generic(cruna_ctx *c, const double *q_in, double *rhs, double *qbc, int bc_mask) {
+  if (c->march_y_ok) {
+    rhs_direct_march_y(c, q_in, rhs, qbc, bc_mask, 0, nullptr, nullptr, nullptr, 0.0);
+    return;
+  }
+  if (c->dir_ok) {
+    rhs_direct_dir(c, q_in, rhs, qbc, bc_mask, 0, nullptr, nullptr, nullptr, 0.0);
+    return;
+  }
   const long long N = c->g.N;
   double *t = c->tmp;
   auto F = [&](int f) { return t + (long long)f * N; };
@@ -1092,8 +1015,30 @@ __global__ void k_adj_dir(long long N, int d, int first, const double *__restric
   }
 }
 
+void stage_adjoint_generic(cruna_ctx *c, const double *qs, const double *q, const double *g, double *k, double *qsbc,
+                           int stage, const double *qs0, double *acc, double *qnext, double dt) {
+  if (c->march_y_ok) {
+    rhs_adjoint_march_y(c, qs, q, g, k, qsbc, stage, qs0, acc, qnext, dt);
+    return;
+  }
+  if (c->dir_ok) {
+    rhs_adjoint_dir(c, qs, q, g, k, qsbc, stage, qs0, acc, qnext, dt);
+    return;
+  }
+  rhs_adjoint_generic(c, qs, q, g, k, qsbc);
+  rk_stage(c, stage, dt, k, qs0, acc, qnext);
+}
+
 void rhs_adjoint_generic(cruna_ctx *c, const double *qs_in, const double *q, const double *g, double *rhs,
                          double *qsbc) {
+  if (c->march_y_ok) {
+    rhs_adjoint_march_y(c, qs_in, q, g, rhs, qsbc, 0, nullptr, nullptr, nullptr, 0.0);
+    return;
+  }
+  if (c->dir_ok) {
+    rhs_adjoint_dir(c, qs_in, q, g, rhs, qsbc, 0, nullptr, nullptr, nullptr, 0.0);
+    return;
+  }
   const long long N = c->g.N;
   double *t = c->tmp;
   auto F = [&](int f) { return t + (long long)f * N; };

@@ -103,6 +103,60 @@ bool diff_is_periodic(int scheme) {
          scheme == CRUNA_DIFF_O6_I_C_P || scheme == CRUNA_DIFF_O8_E_C_P;
 }
 
+bool build_line_table(int n, const std::vector<double> &dl, const std::vector<double> &d, const std::vector<double> &du,
+                      const std::vector<double> &fbnorm, std::vector<double> &tab, int &kf, int &kb) {
+  if (n < 1 || n > kLineMaxN) return false;
+  constexpr int L = kLineL;
+  const int C = (n + L - 1) / L, rows = C * L;
+  std::vector<double> l(rows, 0.0), u(rows, 1.0), c(rows, 0.0);
+  for (int i = 0; i < n; ++i) {
+    if (i > 0) l[i] = dl[i - 1] / u[i - 1];
+    u[i] = i > 0 ? d[i] - l[i] * du[i - 1] : d[i];
+    // the schemes' matrices keep every pivot above 0.1 of their unit-size diagonal
+    if (!(std::fabs(u[i]) > 1e-3) || !(std::fabs(l[i]) < 1e2)) return false;
+    if (i < n - 1) c[i] = du[i] / u[i];
+  }
+  tab.assign((size_t)rows * 6, 0.0);
+  std::vector<double> pf(C, 0.0), qb(C, 0.0);
+  for (int b = 0; b < C; ++b) {
+    double p = 1.0;
+    for (int i = b * L; i < (b + 1) * L; ++i) {
+      p *= -l[i];
+      double *r = &tab[(size_t)i * 6];
+      r[0] = l[i];
+      r[1] = p;
+      r[2] = i < n ? 1.0 / u[i] : 0.0;
+      r[3] = c[i];
+      r[5] = i < n && !fbnorm.empty() ? fbnorm[i] : 0.0;
+    }
+    pf[b] = std::fabs(p);
+    p = 1.0;
+    for (int i = (b + 1) * L - 1; i >= b * L; --i) {
+      p *= -c[i];
+      tab[(size_t)i * 6 + 4] = p;
+    }
+    qb[b] = std::fabs(p);
+  }
+  // smallest number of chunk ends after which the factor on an older one is below 1e-20, for every chunk
+  auto look = [&](const std::vector<double> &f, bool forward) {
+    int need = 1;
+    for (int b = 0; b < C; ++b) {
+      double p = 1.0;
+      int k = 0;
+      for (int j = forward ? b - 1 : b + 1; j >= 0 && j < C; j += forward ? -1 : 1) {
+        ++k;
+        p *= f[j];
+        if (p < 1e-20) break;
+      }
+      need = k > need ? k : need;
+    }
+    return need;
+  };
+  kf = look(pf, true);
+  kb = look(qb, false);
+  return true;
+}
+
 static void set_row(LineOp &op, int row, std::initializer_list<double> w) {
   int m = 0;
   for (double v : w) op.brow[row][m++] = v;

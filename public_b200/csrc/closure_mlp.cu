@@ -51,7 +51,7 @@ struct FwdSmem {
   __nv_bfloat16 X[128 * 16];
   __nv_bfloat16 H1[128 * HID];
   __nv_bfloat16 H2[128 * HID];
-  float b1[HID], b2[HID], b3[16];
+  alignas(16) float b1[HID], b2[HID], b3[16];
   uint64_t mbar;
   uint32_t tmem;
 };
@@ -116,8 +116,7 @@ __global__ void __launch_bounds__(128) k_mlp_forward(const float *__restrict__ P
     tc::fence_after();
     for (int c = 0; c < 4; ++c) {
       tc::tmem_ld16(tb + lane + c * 16, v);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = gelu(v[i] + S.b1[c * 16 + i]);
+      gelu16(v, S.b1 + c * 16);
       put8(S.H1, tid, c * 16, 64, v);
       put8(S.H1, tid, c * 16 + 8, 64, v + 8);
     }
@@ -135,8 +134,7 @@ __global__ void __launch_bounds__(128) k_mlp_forward(const float *__restrict__ P
     tc::fence_after();
     for (int c = 0; c < 4; ++c) {
       tc::tmem_ld16(tb + lane + 64 + c * 16, v);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = gelu(v[i] + S.b2[c * 16 + i]);
+      gelu16(v, S.b2 + c * 16);
       put8(S.H2, tid, c * 16, 64, v);
       put8(S.H2, tid, c * 16 + 8, 64, v + 8);
     }

@@ -42,7 +42,7 @@ struct ClSmem {
   __nv_bfloat16 W1[mlp::HID * 16];
   __nv_bfloat16 W2[mlp::HID * mlp::HID];
   __nv_bfloat16 W3[16 * mlp::HID];
-  float b1[mlp::HID], b2[mlp::HID], b3[16];
+  alignas(16) float b1[mlp::HID], b2[mlp::HID], b3[16];
   uint64_t mbar;
   uint32_t tmem;
 };
@@ -342,8 +342,7 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const
       mma(0, clX, cs->W1, 16, 64);
       for (int c = 0; c < 4 && cl_ok; ++c) {
         tc::tmem_ld16(tb + lane + c * 16, v);
-#pragma unroll
-        for (int e = 0; e < 16; ++e) v[e] = mlp::gelu(v[e] + cs->b1[c * 16 + e]);
+        mlp::gelu16(v, cs->b1 + c * 16);
         mlp::put8(clH, tid, c * 16, 64, v);
         mlp::put8(clH, tid, c * 16 + 8, 64, v + 8);
       }
@@ -352,8 +351,7 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const
         // H1 has been consumed by the finished product: H2 takes its place
         for (int c = 0; c < 4; ++c) {
           tc::tmem_ld16(tb + lane + 64 + c * 16, v);
-#pragma unroll
-          for (int e = 0; e < 16; ++e) v[e] = mlp::gelu(v[e] + cs->b2[c * 16 + e]);
+          mlp::gelu16(v, cs->b2 + c * 16);
           mlp::put8(clH, tid, c * 16, 64, v);
           mlp::put8(clH, tid, c * 16 + 8, 64, v + 8);
         }

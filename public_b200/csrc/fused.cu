@@ -60,8 +60,9 @@ constexpr bool cl_alias_plane() { return plane_bytes_g<T, R>() >= kClActBytes; }
 //
 // YX: the y derivatives come from the line engine (compact schemes along y, dir_passes.cu): the tile has no y
 // halos and the pass adds a.yr and reads the gradients of a.yt.
-template <typename T, int R, bool PER, bool CL = false, bool YX = false>
-__global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const __grid_constant__ FusedArgs a) {
+// Z0: an empty z direction (2-D runs): no ring and no z derivatives, so that four blocks fit an SM.
+template <typename T, int R, bool PER, bool CL = false, bool YX = false, bool Z0 = false>
+__global__ void __launch_bounds__(TX *TY, Z0 ? 4 : (sizeof(T) == 4 ? 3 : 2)) k_pass_g(const __grid_constant__ FusedArgs a) {
   constexpr int RY = YX ? 0 : R, NPF = YX ? 6 : 7;
   constexpr int PW = TX + 2 * R, PH = TY + 2 * RY, PS = PW * PH;
   constexpr int NS = ring_slots(R);
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const
     rp[4 * RS] = T(p - a.p_ref);
     rp[5 * RS] = T(rw);
   };
-  for (int kk = k0 - R; kk < k0 + R; ++kk) {
+  for (int kk = k0 - R; !Z0 && kk < k0 + R; ++kk) {
     const int gk = gidx(oz, kk);
     if (gk < 0 || !col) continue;
     const long long pt = colpt + (long long)n12 * gk;
@@ -128,13 +129,13 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const
   double pruv[2] = {0, 0};
   int pf_ok = 0;
   auto prefetch = [&](int kk, int kc) {
-    const int gk = gidx(oz, kk);
+    const int gk = Z0 ? (kc < k1 ? kc : -1) : gidx(oz, kk);
     pf_ok = (gk >= 0 && col);
     if (pf_ok) {
       const long long pt = colpt + (long long)n12 * gk;
       pf[0] = Q0[pt]; pf[1] = Q1[pt]; pf[2] = Q2[pt]; pf[3] = Q3[pt]; pf[4] = Q4[pt];
     }
-    if (col && kc < k1) {
+    if (!Z0 && col && kc < k1) {
       const long long pt = colpt + (long long)n12 * kc;
       pruv[0] = Q1[pt];
       if constexpr (!YX) pruv[1] = Q2[pt];
@@ -158,9 +159,15 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const
   for (int k = k0; k < k1; ++k) {
     T outv[CL ? NG : 1];                               // closure: pass-G outputs held across the network
     float feat[CL ? mlp::IN : 1];
-    if (pf_ok) put_ring(k + R, pf[0], pf[1], pf[2], pf[3], pf[4]);
+    if (!Z0 && pf_ok) put_ring(k + R, pf[0], pf[1], pf[2], pf[3], pf[4]);
     const int slot = k % NS;
-    {
+    if constexpr (Z0) {
+      T *c = plane + (ty + RY) * PW + (tx + R);
+      const double ir = 1.0 / pf[0];
+      c[0 * PS] = T(pf[1] * ir); c[1 * PS] = T(pf[2] * ir); c[2 * PS] = T(pf[3] * ir);
+      c[3 * PS] = T(a.WoR * pf[4] * ir - a.T_ref);
+      c[4 * PS] = T(pf[4] - a.p_ref); c[5 * PS] = T(pf[1]); c[6 * PS] = T(pf[2]);
+    } else {
       T *c = plane + (ty + RY) * PW + (tx + R);
       const T *rp = ring + slot * NRF * RS + tid;
 #pragma unroll
@@ -200,36 +207,45 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const
       const T *c = plane + (ty + RY) * PW + (tx + R);
       const T *U = c, *V = c + PS, *W = c + 2 * PS, *TT = c + 3 * PS, *P = c + 4 * PS, *RU = c + 5 * PS,
               *RV = c + 6 * PS;
-      int so[NS];
-#pragma unroll
-      for (int m = -R; m <= R; ++m) so[m + R] = ((slot + m + NS) % NS) * NRF * RS + tid;
-      auto column = [&](int f, T *v) {
-#pragma unroll
-        for (int m = 0; m < NS; ++m) v[m] = ring[so[m] + f * RS];
-      };
       const T sx = T(ox.scale), sy = T(oy.scale), sz = T(oz.scale);
-      // z derivatives one column at a time (rho*w and w stay for the products)
-      T zrw[NS], zw[NS], zt[NS];
-      column(5, zrw);
-      column(2, zw);
-      const T m3 = Dz1<T, R, PER>(oz, zrw, k) * sz;
-      const T wz = Dz1<T, R, PER>(oz, zw, k) * sz;
-      const T a3z = Dz2<T, R, PER>(oz, zrw, zw, k) * sz;
-      column(0, zt);
-      const T uz = Dz1<T, R, PER>(oz, zt, k) * sz;
-      const T a1z = Dz2<T, R, PER>(oz, zrw, zt, k) * sz;
-      const T uc = zt[R];
-      column(1, zt);
-      const T vz = Dz1<T, R, PER>(oz, zt, k) * sz;
-      const T a2z = Dz2<T, R, PER>(oz, zrw, zt, k) * sz;
-      const T vc = zt[R];
-      column(3, zt);
-      const T tgz = Dz1<T, R, PER>(oz, zt, k) * T(oz.scale_h);
-      const T Tc = zt[R];
-      column(4, zt);
-      const T pz = Dz1<T, R, PER>(oz, zt, k) * sz;
-      const T ezp = Dz2<T, R, PER>(oz, zt, zw, k) * sz;
-      const T wc = zw[R];
+      T m3 = T(0), wz = T(0), a3z = T(0), uz = T(0), a1z = T(0), vz = T(0), a2z = T(0), tgz = T(0), pz = T(0), ezp = T(0);
+      T uc, vc, wc, Tc;
+      if constexpr (Z0) {
+        uc = U[0];
+        vc = V[0];
+        wc = W[0];
+        Tc = TT[0];
+      } else {
+        int so[NS];
+#pragma unroll
+        for (int m = -R; m <= R; ++m) so[m + R] = ((slot + m + NS) % NS) * NRF * RS + tid;
+        auto column = [&](int f, T *v) {
+#pragma unroll
+          for (int m = 0; m < NS; ++m) v[m] = ring[so[m] + f * RS];
+        };
+        // z derivatives one column at a time (rho*w and w stay for the products)
+        T zrw[NS], zw[NS], zt[NS];
+        column(5, zrw);
+        column(2, zw);
+        m3 = Dz1<T, R, PER>(oz, zrw, k) * sz;
+        wz = Dz1<T, R, PER>(oz, zw, k) * sz;
+        a3z = Dz2<T, R, PER>(oz, zrw, zw, k) * sz;
+        column(0, zt);
+        uz = Dz1<T, R, PER>(oz, zt, k) * sz;
+        a1z = Dz2<T, R, PER>(oz, zrw, zt, k) * sz;
+        uc = zt[R];
+        column(1, zt);
+        vz = Dz1<T, R, PER>(oz, zt, k) * sz;
+        a2z = Dz2<T, R, PER>(oz, zrw, zt, k) * sz;
+        vc = zt[R];
+        column(3, zt);
+        tgz = Dz1<T, R, PER>(oz, zt, k) * T(oz.scale_h);
+        Tc = zt[R];
+        column(4, zt);
+        pz = Dz1<T, R, PER>(oz, zt, k) * sz;
+        ezp = Dz2<T, R, PER>(oz, zt, zw, k) * sz;
+        wc = zw[R];
+      }
       // velocity gradients (ns_rho_rhou_p.f90:102-112) and temperature gradient (:189-191)
       const T ux = D1<T, R, PER>(ox, U, 1, i) * sx, vx = D1<T, R, PER>(ox, V, 1, i) * sx;
       const T wx = D1<T, R, PER>(ox, W, 1, i) * sx;
@@ -398,8 +414,9 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_pass_g(const
 // ------------------------------------------------------------------------------------------------
 // YX: without the y derivatives, which the line engine has added to the convective terms already (plane fields
 // 0 t11, 1 t12, 2 t13, 3 hx, no y halos)
-template <typename T, int R, bool PER, bool YX = false>
-__global__ void __launch_bounds__(TX *TY, 3) k_pass_d(const __grid_constant__ FusedArgs a) {
+// Z0: an empty z direction (2-D runs), no ring.
+template <typename T, int R, bool PER, bool YX = false, bool Z0 = false>
+__global__ void __launch_bounds__(TX *TY, Z0 ? 4 : 3) k_pass_d(const __grid_constant__ FusedArgs a) {
   constexpr int RY = YX ? 0 : R, NPF = YX ? 4 : 7;
   constexpr int PW = TX + 2 * R, PH = TY + 2 * RY, PS = PW * PH;
   constexpr int NS = ring_slots(R);
@@ -424,7 +441,7 @@ __global__ void __launch_bounds__(TX *TY, 3) k_pass_d(const __grid_constant__ Fu
   HaloSet<R, RY> hs;
   hs.init(ox, oy, i0, j0, tid, n1);
 
-  for (int kk = k0 - R; kk < k0 + R; ++kk) {
+  for (int kk = k0 - R; !Z0 && kk < k0 + R; ++kk) {
     const int gk = gidx(oz, kk);
     if (gk < 0 || !col) continue;
     const long long pt = colpt + (long long)n12 * gk;
@@ -437,7 +454,7 @@ __global__ void __launch_bounds__(TX *TY, 3) k_pass_d(const __grid_constant__ Fu
   int pf_ok = 0;
   auto prefetch = [&](int kk, int kc) {
     const int gk = gidx(oz, kk);
-    pf_ok = (gk >= 0 && col);
+    pf_ok = (!Z0 && gk >= 0 && col);
     if (pf_ok) {
       const long long pt = colpt + (long long)n12 * gk;
 #pragma unroll
@@ -510,23 +527,26 @@ __global__ void __launch_bounds__(TX *TY, 3) k_pass_d(const __grid_constant__ Fu
     if (inside) {
       const int i = i0 + tx, j = j0 + ty;
       const T *c = plane + (ty + RY) * PW + (tx + R);
-      int so[NS];
-#pragma unroll
-      for (int m = -R; m <= R; ++m) so[m + R] = ((slot + m + NS) % NS) * NRF * RS + tid;
-      T zc[NS];
       const T sx = T(ox.scale), sy = T(oy.scale), sz = T(oz.scale);
+      T v1z = T(0), v2z = T(0), v3z = T(0), qz = T(0);
+      if constexpr (!Z0) {
+        int so[NS];
 #pragma unroll
-      for (int m = 0; m < NS; ++m) zc[m] = ring[so[m] + 0 * RS];
-      const T v1z = Dz1<T, R, PER>(oz, zc, k) * sz;               // d_z tau_13
+        for (int m = -R; m <= R; ++m) so[m + R] = ((slot + m + NS) % NS) * NRF * RS + tid;
+        T zc[NS];
 #pragma unroll
-      for (int m = 0; m < NS; ++m) zc[m] = ring[so[m] + 1 * RS];
-      const T v2z = Dz1<T, R, PER>(oz, zc, k) * sz;               // d_z tau_23
+        for (int m = 0; m < NS; ++m) zc[m] = ring[so[m] + 0 * RS];
+        v1z = Dz1<T, R, PER>(oz, zc, k) * sz;               // d_z tau_13
 #pragma unroll
-      for (int m = 0; m < NS; ++m) zc[m] = ring[so[m] + 2 * RS];
-      const T v3z = Dz1<T, R, PER>(oz, zc, k) * sz;               // d_z tau_33
+        for (int m = 0; m < NS; ++m) zc[m] = ring[so[m] + 1 * RS];
+        v2z = Dz1<T, R, PER>(oz, zc, k) * sz;               // d_z tau_23
 #pragma unroll
-      for (int m = 0; m < NS; ++m) zc[m] = ring[so[m] + 3 * RS];
-      const T qz = Dz1<T, R, PER>(oz, zc, k) * T(oz.scale_h);     // d_z (lambda d_z T)
+        for (int m = 0; m < NS; ++m) zc[m] = ring[so[m] + 2 * RS];
+        v3z = Dz1<T, R, PER>(oz, zc, k) * sz;               // d_z tau_33
+#pragma unroll
+        for (int m = 0; m < NS; ++m) zc[m] = ring[so[m] + 3 * RS];
+        qz = Dz1<T, R, PER>(oz, zc, k) * T(oz.scale_h);     // d_z (lambda d_z T)
+      }
       const T v1x = D1<T, R, PER>(ox, c + 0 * PS, 1, i) * sx;     // d_x tau_11
       const T v2x = D1<T, R, PER>(ox, c + 1 * PS, 1, i) * sx;     // d_x tau_21
       const T v3x = D1<T, R, PER>(ox, c + 2 * PS, 1, i) * sx;     // d_x tau_31
@@ -646,6 +666,27 @@ void launch_passes(cruna_ctx *c, FusedArgs &a) {
     CRUNA_LAUNCH_CHECK(c);
   }
 }
+
+// 2-D runs: x and y periodic o8, z empty, FP64.  Vortex 256^2: pass G 30 -> 10.4 us, pass D 17 -> 7.7 us (one wave of
+// blocks at four an SM, periodic evaluators in place of the run-time operators).
+void launch_z0(cruna_ctx *c, FusedArgs &a) {
+  constexpr int R = 4;
+  constexpr size_t sm = sizeof(double) * 7 * (TX + 2 * R) * (TY + 2 * R);
+  const dim3 grid((c->g.n1 + TX - 1) / TX, (c->g.n2 + TY - 1) / TY, c->g.n3);
+  a.kc = 1;
+  {
+    ProfScope ps(c, "pass_g");
+    k_pass_g<double, R, true, false, false, true><<<grid, dim3(TX, TY), sm, c->stream>>>(a);
+    CRUNA_LAUNCH_CHECK(c);
+  }
+  {
+    ProfScope ps(c, "pass_d");
+    k_pass_d<double, R, true, false, true><<<grid, dim3(TX, TY), sm, c->stream>>>(a);
+    CRUNA_LAUNCH_CHECK(c);
+  }
+}
+
+bool periodic_o8(const LineOp &op) { return op.kind == OP_STENCIL && !op.solve && op.periodic && op.r == 4; }
 
 template <typename T>
 void launch_for(cruna_ctx *c, FusedArgs &a, int R, bool per) {
@@ -769,7 +810,10 @@ void rhs_direct_fused(cruna_ctx *c, const double *q_in, double *rhs, int stage, 
   const int Rl = R <= 2 ? 2 : 4;
   bool per = true;
   for (int d = 0; d < 3; ++d) per = per && c->dop[d].kind == OP_STENCIL && c->dop[d].periodic && c->dop[d].r == Rl;
-  if (fp32) launch_for<float>(c, a, R, per);
+  if (!fp32 && !a.cl_P && c->g.n3 <= 65535 && periodic_o8(c->dop[0]) && periodic_o8(c->dop[1]) &&
+      c->dop[2].kind == OP_ZERO)
+    launch_z0(c, a);
+  else if (fp32) launch_for<float>(c, a, R, per);
   else launch_for<double>(c, a, R, per);
   if (stage == 0 || split) {
     if (c->has_rhs_bc) bc_rhs(c, rhs, q);                          // :218

@@ -207,21 +207,23 @@ __device__ __forceinline__ bool step_wait(GradSmem &S, uint32_t &phase, int &ok)
   return ok;
 }
 
-__global__ void __launch_bounds__(128, 1) k_mlp_grad(const float *__restrict__ P, const __grid_constant__ Scaling sc,
+__global__ void __launch_bounds__(256, 1) k_mlp_grad(const float *__restrict__ P, const __grid_constant__ Scaling sc,
                                                      const float *__restrict__ X, const float *__restrict__ Yt,
                                                      const int *__restrict__ idx, int batch,
                                                      float *__restrict__ partial, int *err) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   GradSmem &S = *reinterpret_cast<GradSmem *>(smem_raw);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  // two threads a sample: both warpgroups reach the TMEM lanes of their warps' quarter, each takes half the columns
+  const int half = threadIdx.x >> 7, tid = threadIdx.x & 127, warp = tid >> 5;
   stage_weights(P, S.W1, S.W2, S.W3, S.W3T, S.W2T);
-  if (tid < HID) {
+  if (half == 0 && tid < HID) {
     S.b1[tid] = P[OB1 + tid];
     S.b2[tid] = P[OB2 + tid];
   }
-  if (tid < 16) S.b3[tid] = tid < OUT ? P[OB3 + tid] : 0.0f;
+  if (half == 0 && tid < 16) S.b3[tid] = tid < OUT ? P[OB3 + tid] : 0.0f;
   const __nv_bfloat16 zero = __float2bfloat16_rn(0.0f), one = __float2bfloat16_rn(1.0f);
-  for (int s = tid; s < 128; s += 128) {  // constant rows: ones and zero padding
+  if (half == 0) {  // constant rows: ones and zero padding
+    const int s = tid;
     for (int r = 12; r < 16; ++r) S.XT[tc::kmaj(r, s, 128)] = r == 12 ? one : zero;
     for (int r = 64; r < 80; ++r) {
       S.H1T[tc::kmaj(r, s, 128)] = r == 64 ? one : zero;
@@ -229,8 +231,8 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const float *__restrict__ P
     }
     for (int r = OUT; r < 16; ++r) S.dYT[tc::kmaj(r, s, 128)] = zero;
   }
-  if (tid == 0) tc::mbar_init(&S.mbar, 1);
-  if (warp == 0) tc::tmem_alloc(&S.tmem, 256);
+  if (threadIdx.x == 0) tc::mbar_init(&S.mbar, 1);
+  if (threadIdx.x < 32) tc::tmem_alloc(&S.tmem, 256);
   tc::fence_async_smem();
   tc::fence_before();
   __syncthreads();
@@ -254,20 +256,23 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const float *__restrict__ P
     load_features(X, row, true, sc, v);
 #pragma unroll
     for (int o = 0; o < OUT; ++o) t[o] = Yt[row * OUT + o] / sc.out_scale[o];
-    put8(S.X, tid, 0, 16, v);
-    put8(S.X, tid, 8, 16, v + 8);
+    if (half == 0) {
+      put8(S.X, tid, 0, 16, v);
+      put8(S.X, tid, 8, 16, v + 8);
+    } else {
 #pragma unroll
-    for (int f = 0; f < IN; ++f) S.XT[tc::kmaj(f, tid, 128)] = __float2bfloat16_rn(v[f]);
+      for (int f = 0; f < IN; ++f) S.XT[tc::kmaj(f, tid, 128)] = __float2bfloat16_rn(v[f]);
+    }
     tc::fence_async_smem();
     __syncthreads();
-    if (tid == 0) {  // z1 = x W1^T
+    if (threadIdx.x == 0) {  // z1 = x W1^T
       tc::fence_after();
       tc::gemm_bf16(tb + C_A, aX, aW1, 16, 64, false);
       tc::commit(&S.mbar);
     }
     if (!step_wait(S, phase, ok)) break;
     tc::fence_after();
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 2 * half; c < 2 * half + 2; ++c) {
       tc::tmem_ld16(tb + lane + C_A + c * 16, v);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
@@ -284,14 +289,14 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const float *__restrict__ P
     tc::fence_before();
     tc::fence_async_smem();
     __syncthreads();
-    if (tid == 0) {  // z2 = h1 W2^T
+    if (threadIdx.x == 0) {  // z2 = h1 W2^T
       tc::fence_after();
       tc::gemm_bf16(tb + C_B, aH1, aW2, 64, 64, false);
       tc::commit(&S.mbar);
     }
     if (!step_wait(S, phase, ok)) break;
     tc::fence_after();
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 2 * half; c < 2 * half + 2; ++c) {
       tc::tmem_ld16(tb + lane + C_B + c * 16, v);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
@@ -308,7 +313,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const float *__restrict__ P
     tc::fence_before();
     tc::fence_async_smem();
     __syncthreads();
-    if (tid == 0) {  // y = h2 W3^T
+    if (threadIdx.x == 0) {  // y = h2 W3^T
       tc::fence_after();
       tc::gemm_bf16(tb + C_C, aH2, aW3, 64, 16, false);
       tc::commit(&S.mbar);
@@ -316,22 +321,24 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const float *__restrict__ P
     if (!step_wait(S, phase, ok)) break;
     tc::fence_after();
     tc::tmem_ld16(tb + lane + C_C, v);
-    float dy[16];
+    if (half == 0) {
+      float dy[16];
 #pragma unroll
-    for (int o = 0; o < 16; ++o) dy[o] = 0.0f;
+      for (int o = 0; o < 16; ++o) dy[o] = 0.0f;
 #pragma unroll
-    for (int o = 0; o < OUT; ++o) {
-      const float e = v[o] + S.b3[o] - t[o];
-      lsum += e * e;
-      dy[o] = dscale * e;
-      S.dYT[tc::kmaj(o, tid, 128)] = __float2bfloat16_rn(dy[o]);
+      for (int o = 0; o < OUT; ++o) {
+        const float e = v[o] + S.b3[o] - t[o];
+        lsum += e * e;
+        dy[o] = dscale * e;
+        S.dYT[tc::kmaj(o, tid, 128)] = __float2bfloat16_rn(dy[o]);
+      }
+      put8(S.dY, tid, 0, 16, dy);
+      put8(S.dY, tid, 8, 16, dy + 8);
     }
-    put8(S.dY, tid, 0, 16, dy);
-    put8(S.dY, tid, 8, 16, dy + 8);
     tc::fence_before();
     tc::fence_async_smem();
     __syncthreads();
-    if (tid == 0) {  // dH2 = dy W3; [dW3^T | db3] += [h2 | 1]^T dy
+    if (threadIdx.x == 0) {  // dH2 = dy W3; [dW3^T | db3] += [h2 | 1]^T dy
       tc::fence_after();
       tc::gemm_bf16(tb + C_A, adY, aW3T, 16, 64, false);
       tc::gemm_bf16(tb + C_P3, aH2T, adYT, 128, 16, !first);
@@ -339,7 +346,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const float *__restrict__ P
     }
     if (!step_wait(S, phase, ok)) break;
     tc::fence_after();
-    for (int c = 0; c < 4; ++c) {  // dZ2 = dH2 * GELU'(z2), into the H1 array (h1 is done as an A operand)
+    for (int c = 2 * half; c < 2 * half + 2; ++c) {  // dZ2 = dH2 * GELU'(z2), into the H1 array (h1 is done as an A operand)
       tc::tmem_ld16(tb + lane + C_A + c * 16, v);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
@@ -353,7 +360,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const float *__restrict__ P
     tc::fence_before();
     tc::fence_async_smem();
     __syncthreads();
-    if (tid == 0) {  // dH1 = dZ2 W2; [dW2 | db2] += dZ2^T [h1 | 1]
+    if (threadIdx.x == 0) {  // dH1 = dZ2 W2; [dW2 | db2] += dZ2^T [h1 | 1]
       tc::fence_after();
       tc::gemm_bf16(tb + C_B, aH1, aW2T, 64, 64, false);
       tc::gemm_bf16(tb + C_P2, adZ2T, aH1T, 128, 80, !first);
@@ -361,7 +368,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const float *__restrict__ P
     }
     if (!step_wait(S, phase, ok)) break;
     tc::fence_after();
-    for (int c = 0; c < 4; ++c) {  // dZ1 = dH1 * GELU'(z1)
+    for (int c = 2 * half; c < 2 * half + 2; ++c) {  // dZ1 = dH1 * GELU'(z1)
       tc::tmem_ld16(tb + lane + C_B + c * 16, v);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
@@ -372,7 +379,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const float *__restrict__ P
     tc::fence_before();
     tc::fence_async_smem();
     __syncthreads();
-    if (tid == 0) {  // [dW1 | db1] += dZ1^T [x | 1]
+    if (threadIdx.x == 0) {  // [dW1 | db1] += dZ1^T [x | 1]
       tc::fence_after();
       tc::gemm_bf16(tb + C_P1, adZ1T, aXT, 128, 16, !first);
       tc::commit(&S.mbar);
@@ -387,7 +394,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const float *__restrict__ P
     float v[16];
     if (warp < 2) {
       const int j = tid;
-      for (int c = 0; c < 5; ++c) {
+      for (int c = half ? 3 : 0; c < (half ? 5 : 3); ++c) {
         tc::tmem_ld16(tb + lane + C_P2 + c * 16, v);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -396,14 +403,17 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const float *__restrict__ P
           else if (col == HID) out[OB2 + j] = v[i];
         }
       }
-      tc::tmem_ld16(tb + lane + C_P1, v);
+      if (half == 0) {
+        tc::tmem_ld16(tb + lane + C_P1, v);
 #pragma unroll
-      for (int f = 0; f < IN; ++f) out[OW1 + j * IN + f] = v[f];
-      out[OB1 + j] = v[IN];
-      tc::tmem_ld16(tb + lane + C_P3, v);
+        for (int f = 0; f < IN; ++f) out[OW1 + j * IN + f] = v[f];
+        out[OB1 + j] = v[IN];
+      } else {
+        tc::tmem_ld16(tb + lane + C_P3, v);
 #pragma unroll
-      for (int o = 0; o < OUT; ++o) out[OW3 + o * HID + j] = v[o];
-    } else if (warp == 2) {
+        for (int o = 0; o < OUT; ++o) out[OW3 + o * HID + j] = v[o];
+      }
+    } else if (warp == 2 && half == 0) {
       tc::tmem_ld16(tb + lane + C_P3, v);
       if (tid == 64) {
 #pragma unroll
@@ -411,20 +421,20 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(const float *__restrict__ P
       }
     }
   } else if (ok) {  // a CTA without tiles contributes zeros
-    for (int p = tid; p < NPARAMS; p += 128) out[p] = 0.0f;
+    for (int p = threadIdx.x; p < NPARAMS; p += 256) out[p] = 0.0f;
   }
   for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  if ((tid & 31) == 0) S.loss[warp] = lsum;
+  if (half == 0 && (tid & 31) == 0) S.loss[warp] = lsum;
   __syncthreads();
-  if (tid == 0) out[NPARAMS] = ((S.loss[0] + S.loss[1]) + S.loss[2]) + S.loss[3];
+  if (threadIdx.x == 0) out[NPARAMS] = ((S.loss[0] + S.loss[1]) + S.loss[2]) + S.loss[3];
   if (!ok) {
-    if (tid == 0) atomicExch(err, 1);
+    if (threadIdx.x == 0) atomicExch(err, 1);
     tc::mbar_wait(&S.mbar, phase, kWaitLimit);
   }
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
-  if (warp == 0) tc::tmem_free(tb, 256);
+  if (threadIdx.x < 32) tc::tmem_free(tb, 256);
 }
 
 // fixed-order sum of the per-CTA partials: grad[p] = sum_b partial[b][p]; grad[NPARAMS] = loss sum
@@ -436,21 +446,26 @@ __global__ void k_reduce(const float *__restrict__ partial, int nblk, float *__r
   }
 }
 
-// Adam (Kingma & Ba) with bias correction, eps added to sqrt(v_hat)
-__global__ void k_adam(float *__restrict__ P, float *__restrict__ m, float *__restrict__ v,
-                       const float *__restrict__ g, float lr, float b1, float b2, float eps, float c1, float c2) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < NPARAMS; p += gridDim.x * blockDim.x) {
-    const float gp = g[p];
+// one training step's update: the fixed-order sum of the partials, Adam (Kingma & Ba) with bias correction, eps
+// added to sqrt(v_hat), and the step's loss -- one launch where the sum, Adam and the loss took three (10 of
+// 44 us of a step of 4096 samples)
+__global__ void k_update(const float *__restrict__ partial, int nblk, float *__restrict__ P, float *__restrict__ m,
+                         float *__restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2,
+                         float inv_count, float *__restrict__ hist, int step) {
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p <= NPARAMS; p += gridDim.x * blockDim.x) {
+    float gp = 0.0f;
+#pragma unroll 16
+    for (int b = 0; b < nblk; ++b) gp += partial[(long long)b * (NPARAMS + 1) + p];
+    if (p == NPARAMS) {
+      hist[step] = gp * inv_count;
+      continue;
+    }
     const float mp = b1 * m[p] + (1.0f - b1) * gp;
     const float vp = b2 * v[p] + (1.0f - b2) * gp * gp;
     m[p] = mp;
     v[p] = vp;
     P[p] -= lr * (mp / c1) / (sqrtf(vp / c2) + eps);
   }
-}
-
-__global__ void k_loss_store(const float *__restrict__ grad, float inv_count, float *__restrict__ hist, int step) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) hist[step] = grad[NPARAMS] * inv_count;
 }
 
 }  // namespace mlp
@@ -536,13 +551,19 @@ void ensure_idx(cruna_mlp *h, long long n) {
   h->idx_cap = n;
 }
 
-// one gradient evaluation of the batch idx[0 .. batch): grad (+ loss sum at NPARAMS)
-void run_grad(cruna_mlp *h, const float *X, const float *Y, const int *idx, int batch) {
+// per-CTA partial gradients of the batch idx[0 .. batch); returns the number of CTAs
+int run_partials(cruna_mlp *h, const float *X, const float *Y, const int *idx, int batch) {
   set_attrs(h);
   const int tiles = batch / 128;
   const int nblk = std::min(tiles, sm_count(h->device));
-  k_mlp_grad<<<nblk, 128, sizeof(GradSmem), h->stream>>>(h->P, h->sc, X, Y, idx, batch, h->partial, h->flag);
+  k_mlp_grad<<<nblk, 256, sizeof(GradSmem), h->stream>>>(h->P, h->sc, X, Y, idx, batch, h->partial, h->flag);
   ck(cudaGetLastError(), "k_mlp_grad launch");
+  return nblk;
+}
+
+// one gradient evaluation: grad (+ loss sum at NPARAMS)
+void run_grad(cruna_mlp *h, const float *X, const float *Y, const int *idx, int batch) {
+  const int nblk = run_partials(h, X, Y, idx, batch);
   k_reduce<<<(NPARAMS + 256) / 256, 256, 0, h->stream>>>(h->partial, nblk, h->grad);
   ck(cudaGetLastError(), "k_reduce launch");
 }
@@ -727,13 +748,12 @@ int cruna_mlp_train_dev(cruna_mlp *h, const float *X, const float *Y, long long 
            "indices");
         ck(cudaStreamSynchronize(h->stream), "sync");
       }
-      run_grad(h, X, Y, h->idx + e * batch, batch);
+      const int nblk = run_partials(h, X, Y, h->idx + e * batch, batch);
       ++h->adam_t;
       const float c1 = 1.0f - std::pow(b1, (float)h->adam_t), c2 = 1.0f - std::pow(b2, (float)h->adam_t);
-      k_adam<<<(NPARAMS + 255) / 256, 256, 0, h->stream>>>(h->P, h->m, h->v, h->grad, lr, b1, b2, eps, c1, c2);
-      ck(cudaGetLastError(), "k_adam launch");
-      k_loss_store<<<1, 32, 0, h->stream>>>(h->grad, 1.0f / ((float)batch * OUT), h->hist, s);
-      ck(cudaGetLastError(), "k_loss_store launch");
+      k_update<<<(NPARAMS + 128) / 128, 128, 0, h->stream>>>(h->partial, nblk, h->P, h->m, h->v, lr, b1, b2, eps, c1, c2,
+                                                             1.0f / ((float)batch * OUT), h->hist, s);
+      ck(cudaGetLastError(), "k_update launch");
     }
     if (loss_hist && steps > 0)
       ck(cudaMemcpyAsync(loss_hist, h->hist, sizeof(float) * steps, cudaMemcpyDeviceToHost, h->stream), "losses");

@@ -75,6 +75,7 @@ struct LineOpT {
   const double *band = nullptr;
   int solve = 0;
   LineOp sop;
+  LineOp op;            // the operator itself: away from the ends A^T is its mirrored interior stencil
 };
 
 struct Grid {
@@ -201,7 +202,8 @@ namespace cruna {
 // launch helpers (ops.cu)
 void launch_line_stencil(cruna_ctx *c, const LineOp &op, int dir, const double *f1, const double *f2,
                          double *out, double scale, int nfields, double sign = 1.0);
-void launch_line_solve(cruna_ctx *c, const LineOp &op, int dir, double *data, int nfields);
+// B out = in (out may be in)
+void launch_line_solve(cruna_ctx *c, const LineOp &op, int dir, const double *in, double *out, int nfields);
 void apply_diff(cruna_ctx *c, int dir, const double *f1, const double *f2, double *out, double h,
                 int nfields);
 void apply_filter(cruna_ctx *c, int dir, double *q, double *scratch, int nfields);

@@ -70,6 +70,7 @@ void build_transpose(cruna_ctx *c, const LineOp &op, const HostFactors &hf, Line
   t = LineOpT();
   t.n = op.n;
   t.kind = op.kind;
+  t.op = op;
   if (op.kind != OP_STENCIL) return;
   const int n = op.n;
   const int W = std::max(op.r, op.bw);
@@ -161,34 +162,60 @@ __global__ void k_band_T(LineOpT op, Grid g, int dir, const double *__restrict__
   }
 }
 
-// the same banded product with the line position from the launch grid (x = block x range, y = j,
-// (k, field) = z, strided) instead of a division per point; DIR is compile-time
+// The same product with the line position from the launch grid (x = block x range, y = j, (k, field) = z,
+// strided).  Rows that no closure row and no wrap reaches take the interior stencil mirrored (A^T = -A for
+// derivatives, A for filters there) from constant coefficients with their loads unrolled; the others the band.
+// Mixing layer 128 x 96 x 64, five fields: 53 us with the band throughout, 36 now.
 template <int DIR>
-__global__ void __launch_bounds__(128) k_band_T_grid(LineOpT op, Grid g, const double *__restrict__ in,
-                                                     double *__restrict__ out, double scale, int nfields,
-                                                     int accumulate) {
+__global__ void __launch_bounds__(128) k_band_T_grid(const __grid_constant__ LineOpT op, Grid g,
+                                                     const double *__restrict__ in, double *__restrict__ out,
+                                                     double scale, int nfields, int accumulate) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= g.n1) return;
   const int j = blockIdx.y;
-  const int n = op.n, w = op.hi - op.lo + 1;
+  const int n = op.n, w = op.hi - op.lo + 1, r = op.op.r;
+  const int edge = op.periodic ? r : max(op.op.bw, op.op.nb + r);
   const long long n12 = (long long)g.n1 * g.n2;
   const long long s = DIR == 0 ? 1 : (DIR == 1 ? (long long)g.n1 : n12);
   for (int kf = blockIdx.z; kf < g.n3 * nfields; kf += gridDim.z) {
     const int fld = kf / g.n3, k = kf - fld * g.n3;
     const long long p = x + (long long)g.n1 * j + n12 * k;
     const int i = DIR == 0 ? x : (DIR == 1 ? j : k);
-    const double *a = in + (long long)fld * g.N + p - (long long)i * s;  // the line's first point
-    const double *__restrict__ row = op.band + (long long)i * w;
+    const double *q = in + (long long)fld * g.N + p;
     double v = 0.0;
-    for (int o = op.lo; o <= op.hi; ++o) {
-      int jj = i + o;
-      if (op.periodic) {
-        if (jj < 0) jj += n;
-        else if (jj >= n) jj -= n;
-      } else if (jj < 0 || jj >= n) {
-        continue;
+    if (i >= edge && i < n - edge) {
+      double lo[kMaxR], hi[kMaxR];
+#pragma unroll
+      for (int m = 1; m <= kMaxR; ++m) {
+        lo[m - 1] = hi[m - 1] = 0.0;
+        if (m <= r) {
+          lo[m - 1] = q[-m * s];
+          hi[m - 1] = q[m * s];
+        }
       }
-      v += row[o - op.lo] * a[jj * s];
+      if (op.op.antisym) {
+#pragma unroll
+        for (int m = 1; m <= kMaxR; ++m) v += op.op.c[m] * (lo[m - 1] - hi[m - 1]);
+      } else {
+        const double c0 = q[0];
+        v = op.op.c[0] * c0;
+#pragma unroll
+        for (int m = 1; m <= kMaxR; ++m) v += op.op.c[m] * (lo[m - 1] + hi[m - 1]);
+        if (op.op.blend > 0.0) v = c0 - op.op.blend * (c0 - v);
+      }
+    } else {
+      const double *a = q - (long long)i * s;  // the line's first point
+      const double *__restrict__ row = op.band + (long long)i * w;
+      for (int o = op.lo; o <= op.hi; ++o) {
+        int jj = i + o;
+        if (op.periodic) {
+          if (jj < 0) jj += n;
+          else if (jj >= n) jj -= n;
+        } else if (jj < 0 || jj >= n) {
+          continue;
+        }
+        v += row[o - op.lo] * a[jj * s];
+      }
     }
     v *= scale;
     double *o_ = out + (long long)fld * g.N + p;
@@ -211,8 +238,7 @@ void apply_T(cruna_ctx *c, const LineOpT &t, int dir, const double *in, double *
   }
   const double *src = in;
   if (t.solve) {
-    copy_state(c, scratch, in, nfields);
-    launch_line_solve(c, t.sop, dir, scratch, nfields);
+    launch_line_solve(c, t.sop, dir, in, scratch, nfields);
     src = scratch;
   }
   ProfScope ps(c, "band_T");

@@ -331,15 +331,16 @@ void launch_line_stencil(cruna_ctx *c, const LineOp &op, int dir, const double *
   CRUNA_LAUNCH_CHECK(c);
 }
 
-void launch_line_solve(cruna_ctx *c, const LineOp &op, int dir, double *data, int nfields) {
+void launch_line_solve(cruna_ctx *c, const LineOp &op, int dir, const double *in, double *out, int nfields) {
   static const char *names[3] = {"line_solve_x", "line_solve_y", "line_solve_z"};
   ProfScope ps(c, names[dir]);
   if (op.tab && line_grid_ok(c->g)) {
-    for_sets(c, data, nullptr, data, nfields, [&](const FieldSet &fs) { launch_lines<0, false>(c, op, dir, fs, 1.0); });
+    for_sets(c, in, nullptr, out, nfields, [&](const FieldSet &fs) { launch_lines<0, false>(c, op, dir, fs, 1.0); });
     return;
   }
   const long long lines = (c->g.N / op.n) * nfields;
-  k_line_solve<<<nblocks(lines, 128), 128, 0, c->stream>>>(op, c->g, dir, data, nfields);
+  copy_state(c, out, in, nfields);
+  k_line_solve<<<nblocks(lines, 128), 128, 0, c->stream>>>(op, c->g, dir, out, nfields);
   CRUNA_LAUNCH_CHECK(c);
 }
 
@@ -388,7 +389,7 @@ void apply_diff(cruna_ctx *c, int dir, const double *f1, const double *f2, doubl
     return;
   }
   launch_line_stencil(c, op, dir, f1, f2, out, scale, nfields);
-  if (op.kind == OP_STENCIL && op.solve) launch_line_solve(c, op, dir, out, nfields);
+  if (op.kind == OP_STENCIL && op.solve) launch_line_solve(c, op, dir, out, out, nfields);
 }
 
 // filter_i_d in place: compact filters on the line engine, which works in place; the others out of place
@@ -401,7 +402,7 @@ void apply_filter(cruna_ctx *c, int dir, double *q, double *scratch, int nfields
     return;
   }
   launch_line_stencil(c, op, dir, q, nullptr, scratch, 1.0, nfields);
-  if (op.solve) launch_line_solve(c, op, dir, scratch, nfields);
+  if (op.solve) launch_line_solve(c, op, dir, scratch, scratch, nfields);
   CRUNA_CUDA_CHECK(cudaMemcpyAsync(q, scratch, sizeof(double) * c->g.N * nfields,
                                    cudaMemcpyDeviceToDevice, c->stream));
 }

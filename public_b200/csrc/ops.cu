@@ -411,7 +411,7 @@ void apply_filter(cruna_ctx *c, int dir, double *q, double *scratch, int nfields
 // boundary kernels
 // ------------------------------------------------------------------------------------------------
 
-// characteristic_q_k1d (src/boundaries/nonreflecting.f90:46-137) -- aim from `aim` at p + aim_off
+// characteristic_q_k1d (src/boundaries/nonreflecting.f90:46-137) -- aim from `aim` at p + aim_off (type 200)
 __global__ void k_char_q(Box b, Grid g, double k1, double k2, double k3, double gamma, double *q,
                          const double *aim, long long aim_off) {
   const long long tot = b.count();
@@ -467,6 +467,63 @@ __global__ void k_char_rhs(Box b, Grid g, double k1, double k2, double k3, doubl
     char_rhs_point(rv, qv, av, k1, k2, k3, gamma, dt, out);
     for (int v = 0; v < 5; ++v) rhs[p + v * N] = out[v];
   }
+}
+
+// Consecutive type-201 rows in one launch (a launch costs about 5 us whatever the box): row = blockIdx.y.  Rows
+// apply in table order where boxes overlap (edges and corners): the first row that holds a point does all of
+// them there, one after another; the treatment only touches its own point.
+struct CharRows {
+  static constexpr int kMax = 8;
+  int n = 0;
+  Box box[kMax];
+  double k[kMax][3];
+};
+
+__device__ __forceinline__ bool in_box(const Box &b, int i, int j, int k) {
+  return i >= b.is && i <= b.ie && j >= b.js && j <= b.je && k >= b.ks && k <= b.ke;
+}
+
+template <bool ADJ>
+__global__ void k_char_rows(const __grid_constant__ CharRows rows, Grid g, double gamma, double *q, const double *aim) {
+  const int r = blockIdx.y;
+  const Box &b = rows.box[r];
+  const long long tot = b.count(), N = g.N;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot;
+       t += (long long)gridDim.x * blockDim.x) {
+    int i, j, k;
+    const long long p = box_point(b, g, t, i, j, k);
+    bool mine = true;
+    for (int e = 0; e < r; ++e) mine = mine && !in_box(rows.box[e], i, j, k);
+    if (!mine) continue;
+    double v[5], a[5], out[5];
+    for (int c = 0; c < 5; ++c) {
+      v[c] = q[p + c * N];
+      a[c] = aim[p + c * N];
+    }
+    for (int e = r; e < rows.n; ++e) {
+      if (!in_box(rows.box[e], i, j, k)) continue;
+      if (ADJ) char_qs_point(v, a, rows.k[e][0], rows.k[e][1], rows.k[e][2], gamma, out);
+      else char_q_point(v, a, rows.k[e][0], rows.k[e][1], rows.k[e][2], gamma, out);
+      for (int c = 0; c < 5; ++c) v[c] = out[c];
+    }
+    for (int c = 0; c < 5; ++c) q[p + c * N] = v[c];
+  }
+}
+
+// the type-201 rows from position at on (as many as fit one launch); returns the position after them
+template <bool ADJ>
+static size_t launch_char_rows(cruna_ctx *c, size_t at, double *q, const double *aim) {
+  CharRows rows;
+  int blocks = 1;
+  for (; at < c->bc.size() && c->bc[at].type == 201 && rows.n < CharRows::kMax; ++at) {
+    rows.box[rows.n] = box_of(c->bc[at]);
+    for (int d = 0; d < 3; ++d) rows.k[rows.n][d] = c->bc[at].k[d];
+    blocks = std::max(blocks, nblocks(rows.box[rows.n].count()));
+    ++rows.n;
+  }
+  k_char_rows<ADJ><<<dim3(blocks, rows.n), kThreads, 0, c->stream>>>(rows, c->g, c->cfg.gamma, q, aim);
+  CRUNA_LAUNCH_CHECK(c);
+  return at;
 }
 
 // zonal variants with a normal vector per point (nonreflecting.f90:141-233, :345-449, :558-661): types
@@ -617,16 +674,17 @@ __global__ void k_sponge(int mode, Grid g, SpongeDev sp, double gamma, double *a
 
 void bc_q(cruna_ctx *c, double *q, int outside) {
   ProfScope ps(c, "boundary");
-  for (const BCRow &r : c->bc) {
+  for (size_t at = 0; at < c->bc.size(); ++at) {
+    const BCRow &r = c->bc[at];
+    if (r.type == 201) {
+      at = launch_char_rows<false>(c, at, q, c->qref) - 1;
+      continue;
+    }
     Box b = box_of(r);
     const int blocks = nblocks(b.count());
     if (r.type == 200) {
       k_char_q<<<blocks, kThreads, 0, c->stream>>>(b, c->g, r.k[0], r.k[1], r.k[2], c->cfg.gamma, q, q,
                                                    offset_of(c, r.shift));
-      CRUNA_LAUNCH_CHECK(c);
-    } else if (r.type == 201) {
-      k_char_q<<<blocks, kThreads, 0, c->stream>>>(b, c->g, r.k[0], r.k[1], r.k[2], c->cfg.gamma, q,
-                                                   c->qref, 0);
       CRUNA_LAUNCH_CHECK(c);
     } else if (r.type == 401) {
       k_sponge<<<nblocks(c->g.N), kThreads, 0, c->stream>>>(1, c->g, c->sponge, c->cfg.gamma, q, nullptr,
@@ -642,11 +700,16 @@ void bc_q(cruna_ctx *c, double *q, int outside) {
 
 void bc_qs(cruna_ctx *c, double *qs, const double *q, int outside) {
   ProfScope ps(c, "boundary");
-  for (const BCRow &r : c->bc) {
+  for (size_t at = 0; at < c->bc.size(); ++at) {
+    const BCRow &r = c->bc[at];
+    if (r.type == 201) {
+      at = launch_char_rows<true>(c, at, qs, q) - 1;
+      continue;
+    }
     Box b = box_of(r);
     const int blocks = nblocks(b.count());
-    if (r.type == 200 || r.type == 201) {
-      const long long off = r.type == 200 ? offset_of(c, r.shift) : 0;
+    if (r.type == 200) {
+      const long long off = offset_of(c, r.shift);
       k_char_qs<<<blocks, kThreads, 0, c->stream>>>(b, c->g, r.k[0], r.k[1], r.k[2], c->cfg.gamma, qs, q,
                                                     off);
       CRUNA_LAUNCH_CHECK(c);

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(TX *TY, Z0 ? 4 : (sizeof(T) == 4 ? 3 : 2)) k_p
   for (int kk = k0 - R; !Z0 && kk < k0 + R; ++kk) {
     const int gk = gidx(oz, kk);
     if (gk < 0 || !col) continue;
-    const long long pt = colpt + (long long)n12 * gk;
+    const int pt = colpt + n12 * gk;
     put_ring(kk, Q0[pt], Q1[pt], Q2[pt], Q3[pt], Q4[pt]);
   }
   double pf[5] = {1, 0, 0, 0, 0};
@@ -132,11 +132,11 @@ __global__ void __launch_bounds__(TX *TY, Z0 ? 4 : (sizeof(T) == 4 ? 3 : 2)) k_p
     const int gk = Z0 ? (kc < k1 ? kc : -1) : gidx(oz, kk);
     pf_ok = (gk >= 0 && col);
     if (pf_ok) {
-      const long long pt = colpt + (long long)n12 * gk;
+      const int pt = colpt + n12 * gk;
       pf[0] = Q0[pt]; pf[1] = Q1[pt]; pf[2] = Q2[pt]; pf[3] = Q3[pt]; pf[4] = Q4[pt];
     }
     if (!Z0 && col && kc < k1) {
-      const long long pt = colpt + (long long)n12 * kc;
+      const int pt = colpt + n12 * kc;
       pruv[0] = Q1[pt];
       if constexpr (!YX) pruv[1] = Q2[pt];
     }
@@ -146,11 +146,11 @@ __global__ void __launch_bounds__(TX *TY, Z0 ? 4 : (sizeof(T) == 4 ? 3 : 2)) k_p
   constexpr int NHT = HaloSet<R, RY>::PER_THREAD;
   double hv[NHT][5];
   auto halo_fetch = [&](int kk) {
-    const long long kofs = (long long)n12 * kk;
+    const int kofs = n12 * kk;
 #pragma unroll
     for (int h = 0; h < NHT; ++h) {
       if (hs.goff[h] < 0) continue;
-      const long long pt = hs.goff[h] + kofs;
+      const int pt = hs.goff[h] + kofs;
       hv[h][0] = Q0[pt]; hv[h][1] = Q1[pt]; hv[h][2] = Q2[pt]; hv[h][3] = Q3[pt]; hv[h][4] = Q4[pt];
     }
   };
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(TX *TY, Z0 ? 4 : (sizeof(T) == 4 ? 3 : 2)) k_p
       c[5 * PS] = T(pruv[0]);
       if constexpr (!YX) c[6 * PS] = T(pruv[1]);
     }
-    const long long kofs = (long long)n12 * k;
+    const int kofs = n12 * k;
 #pragma unroll
     for (int h = 0; h < NHT; ++h) {
       if (hs.goff[h] < 0) continue;
@@ -192,13 +192,13 @@ __global__ void __launch_bounds__(TX *TY, Z0 ? 4 : (sizeof(T) == 4 ? 3 : 2)) k_p
     double yd[YX ? 9 : 1];                             // u_y, v_y, w_y, T_y and the y part of the convective terms
     if constexpr (YX) {
       if (inside) {
-        const long long pt = colpt + kofs;
-        yd[0] = a.yt[pt + F_UY * N];
-        yd[1] = a.yt[pt + F_VY * N];
-        yd[2] = a.yt[pt + F_WY * N];
-        yd[3] = a.yt[pt + F_TY * N];
+        const int pt = colpt + kofs;
+        yd[0] = (a.yt + F_UY * N)[pt];
+        yd[1] = (a.yt + F_VY * N)[pt];
+        yd[2] = (a.yt + F_WY * N)[pt];
+        yd[3] = (a.yt + F_TY * N)[pt];
 #pragma unroll
-        for (int v = 0; v < 5; ++v) yd[4 + v] = a.yr[pt + v * N];
+        for (int v = 0; v < 5; ++v) yd[4 + v] = (a.yr + v * N)[pt];
       }
     }
     __syncthreads();
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(TX *TY, Z0 ? 4 : (sizeof(T) == 4 ? 3 : 2)) k_p
       } else {
         int so[NS];
 #pragma unroll
-        for (int m = -R; m <= R; ++m) so[m + R] = ((slot + m + NS) % NS) * NRF * RS + tid;
+        for (int m = -R; m <= R; ++m) so[m + R] = ring_slot<NS>(slot + m) * NRF * RS + tid;
         auto column = [&](int f, T *v) {
 #pragma unroll
           for (int m = 0; m < NS; ++m) v[m] = ring[so[m] + f * RS];
@@ -319,14 +319,14 @@ __global__ void __launch_bounds__(TX *TY, Z0 ? 4 : (sizeof(T) == 4 ? 3 : 2)) k_p
         const double gm = sqrt(g2), ginv = gm > 0.0 ? 1.0 / gm : 0.0;
 #pragma unroll
         for (int f = 0; f < 9; ++f) feat[f] = (float)(a.cl_norm ? gr[f] * ginv : gr[f]);
-        feat[9] = (float)a.q[i + (long long)n1 * j + kofs];
+        feat[9] = (float)a.q[i + n1 * j + kofs];
         feat[10] = (float)Tabs;
         feat[11] = (float)(a.cl_norm ? gm * a.cl_delta : a.cl_delta);
       } else {
         T *go = static_cast<T *>(a.gbuf);
-        const long long pt = i + (long long)n1 * j + kofs;
+        const int pt = i + n1 * j + kofs;
 #pragma unroll
-        for (int f = 0; f < NG; ++f) go[pt + f * N] = o[f];
+        for (int f = 0; f < NG; ++f) (go + f * N)[pt] = o[f];
       }
     }
     if constexpr (CL) {
@@ -388,9 +388,9 @@ __global__ void __launch_bounds__(TX *TY, Z0 ? 4 : (sizeof(T) == 4 ? 3 : 2)) k_p
         outv[9] = T(double(outv[9]) - tm[5]);    // t23
         outv[10] = T(double(outv[10]) - tm[2]);  // t33
         T *go = static_cast<T *>(a.gbuf);
-        const long long pt = (i0 + tx) + (long long)n1 * (j0 + ty) + kofs;
+        const int pt = (i0 + tx) + n1 * (j0 + ty) + kofs;
 #pragma unroll
-        for (int f = 0; f < NG; ++f) go[pt + f * N] = outv[f];
+        for (int f = 0; f < NG; ++f) (go + f * N)[pt] = outv[f];
       }
       if (!cl_ok) break;
     }
@@ -444,10 +444,10 @@ __global__ void __launch_bounds__(TX *TY, Z0 ? 4 : 3) k_pass_d(const __grid_cons
   for (int kk = k0 - R; !Z0 && kk < k0 + R; ++kk) {
     const int gk = gidx(oz, kk);
     if (gk < 0 || !col) continue;
-    const long long pt = colpt + (long long)n12 * gk;
+    const int pt = colpt + n12 * gk;
     T *rp = ring + (((kk % NS) + NS) % NS) * NRF * RS + tid;
 #pragma unroll
-    for (int f = 0; f < NRF; ++f) rp[f * RS] = G[pt + rfld[f] * N];
+    for (int f = 0; f < NRF; ++f) rp[f * RS] = (G + rfld[f] * N)[pt];
   }
   T pf[NRF];
   T pc[NPF];
@@ -456,27 +456,27 @@ __global__ void __launch_bounds__(TX *TY, Z0 ? 4 : 3) k_pass_d(const __grid_cons
     const int gk = gidx(oz, kk);
     pf_ok = (!Z0 && gk >= 0 && col);
     if (pf_ok) {
-      const long long pt = colpt + (long long)n12 * gk;
+      const int pt = colpt + n12 * gk;
 #pragma unroll
-      for (int f = 0; f < NRF; ++f) pf[f] = G[pt + rfld[f] * N];
+      for (int f = 0; f < NRF; ++f) pf[f] = (G + rfld[f] * N)[pt];
     }
     if (col && kc < k1) {
-      const long long pt = colpt + (long long)n12 * kc;
+      const int pt = colpt + n12 * kc;
 #pragma unroll
-      for (int f = 0; f < NPF; ++f) pc[f] = G[pt + pfld[f] * N];
+      for (int f = 0; f < NPF; ++f) pc[f] = (G + pfld[f] * N)[pt];
     }
   };
   prefetch(k0 + R, k0);
   constexpr int NHT = HaloSet<R, RY>::PER_THREAD;
   T hv[NHT][NPF];
   auto halo_fetch = [&](int kk) {
-    const long long kofs = (long long)n12 * kk;
+    const int kofs = n12 * kk;
 #pragma unroll
     for (int h = 0; h < NHT; ++h) {
       if (hs.goff[h] < 0) continue;
-      const long long pt = hs.goff[h] + kofs;
+      const int pt = hs.goff[h] + kofs;
 #pragma unroll
-      for (int f = 0; f < NPF; ++f) hv[h][f] = G[pt + pfld[f] * N];
+      for (int f = 0; f < NPF; ++f) hv[h][f] = (G + pfld[f] * N)[pt];
     }
   };
   halo_fetch(k0);
@@ -492,26 +492,26 @@ __global__ void __launch_bounds__(TX *TY, Z0 ? 4 : 3) k_pass_d(const __grid_cons
 #pragma unroll
       for (int f = 0; f < NPF; ++f) c[f * PS] = pc[f];
     }
-    const long long kofs = (long long)n12 * k;
+    const int kofs = n12 * k;
     // epilogue inputs of this plane, issued before the barrier so their latency overlaps the stencils
-    const long long opt = (i0 + tx) + (long long)n1 * (j0 + ty) + kofs;
+    const int opt = (i0 + tx) + n1 * (j0 + ty) + kofs;
     T e_g[6];
     double e_f[5] = {0, 0, 0, 0, 0}, e_q0[5] = {0, 0, 0, 0, 0}, e_acc[5] = {0, 0, 0, 0, 0};
     if (inside) {
 #pragma unroll
-      for (int f = 0; f < 5; ++f) e_g[f] = G[opt + f * N];
-      e_g[5] = G[opt + 14 * N];
+      for (int f = 0; f < 5; ++f) e_g[f] = (G + f * N)[opt];
+      e_g[5] = (G + 14 * N)[opt];
       if (a.force) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) e_f[v] = a.force[opt + v * N];
+        for (int v = 0; v < 5; ++v) e_f[v] = (a.force + v * N)[opt];
       }
       if (a.stage != 0) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) e_q0[v] = a.q0[opt + v * N];
+        for (int v = 0; v < 5; ++v) e_q0[v] = (a.q0 + v * N)[opt];
       }
       if (a.stage >= 2) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) e_acc[v] = a.acc[opt + v * N];
+        for (int v = 0; v < 5; ++v) e_acc[v] = (a.acc + v * N)[opt];
       }
     }
 #pragma unroll
@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(TX *TY, Z0 ? 4 : 3) k_pass_d(const __grid_cons
       if constexpr (!Z0) {
         int so[NS];
 #pragma unroll
-        for (int m = -R; m <= R; ++m) so[m + R] = ((slot + m + NS) % NS) * NRF * RS + tid;
+        for (int m = -R; m <= R; ++m) so[m + R] = ring_slot<NS>(slot + m) * NRF * RS + tid;
         T zc[NS];
 #pragma unroll
         for (int m = 0; m < NS; ++m) zc[m] = ring[so[m] + 0 * RS];
@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(TX *TY, Z0 ? 4 : 3) k_pass_d(const __grid_cons
         v3y = D1<T, R, PER>(oy, c + 4 * PS, PW, j) * sy;          // d_y tau_32
         qy = D1<T, R, PER>(oy, c + 6 * PS, PW, j) * T(oy.scale_h);
       }
-      const long long pt = opt;
+      const int pt = opt;
       (void)i; (void)j;
       // assembly in the reference's order (:135, 143-149, 157-163, 171-177, 185-209)
       double r1 = double(e_g[0]);
@@ -581,30 +581,29 @@ __global__ void __launch_bounds__(TX *TY, Z0 ? 4 : 3) k_pass_d(const __grid_cons
           const double sh = sponge_at(a.sponge, a.g, opt);
           if (sh != 0.0) {
 #pragma unroll
-            for (int v = 0; v < 5; ++v) kv[v] = kv[v] - sh * (a.q[opt + v * N] - a.sp_qref[opt + v * N]);
+            for (int v = 0; v < 5; ++v) kv[v] = kv[v] - sh * ((a.q + v * N)[opt] - (a.sp_qref + v * N)[opt]);
           }
         }
       }
       if (a.stage == 0) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) a.rhs[pt + v * N] = kv[v];
+        for (int v = 0; v < 5; ++v) (a.rhs + v * N)[pt] = kv[v];
       } else {
         // RK4 stage update (rk_o4_e.f90:45-50)
         const double dt = a.dt, dth = a.dt * 0.5;
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
-          const long long o = pt + v * N;
           if (a.stage == 1) {
-            a.acc[o] = kv[v];
-            a.qnext[o] = e_q0[v] + dth * kv[v];
+            (a.acc + v * N)[pt] = kv[v];
+            (a.qnext + v * N)[pt] = e_q0[v] + dth * kv[v];
           } else if (a.stage == 2) {
-            a.acc[o] = e_acc[v] + 2.0 * kv[v];
-            a.qnext[o] = e_q0[v] + dth * kv[v];
+            (a.acc + v * N)[pt] = e_acc[v] + 2.0 * kv[v];
+            (a.qnext + v * N)[pt] = e_q0[v] + dth * kv[v];
           } else if (a.stage == 3) {
-            a.acc[o] = e_acc[v] + 2.0 * kv[v];
-            a.qnext[o] = e_q0[v] + dt * kv[v];
+            (a.acc + v * N)[pt] = e_acc[v] + 2.0 * kv[v];
+            (a.qnext + v * N)[pt] = e_q0[v] + dt * kv[v];
           } else {
-            a.qnext[o] = e_q0[v] + dt / 6.0 * (e_acc[v] + kv[v]);
+            (a.qnext + v * N)[pt] = e_q0[v] + dt / 6.0 * (e_acc[v] + kv[v]);
           }
         }
       }
@@ -729,6 +728,7 @@ int halo_of(const LineOp &op) {
 bool closure_in_pass(const cruna_ctx *c) { return c->closure_mlp && c->closure_fused && use_fused(c); }
 
 bool fused_supported(const cruna_ctx *c) {
+  if (c->g.N >= (1LL << 31)) return false;                         // 32-bit point offsets (such a state takes 86 GB)
   for (int d = 0; d < 3; ++d) {
     const LineOp &op = c->dop[d];
     if (op.kind == OP_STENCIL && op.solve) return false;           // compact cores: generic path

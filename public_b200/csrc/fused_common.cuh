@@ -58,6 +58,11 @@ struct FusedArgs {
 };
 
 __host__ __device__ constexpr int ring_slots(int R) { return 2 * R + 1; }
+// slot of plane offset s in (-NS, 2 NS) of a ring of NS planes
+template <int NS>
+__device__ __forceinline__ int ring_slot(int s) {
+  return s < 0 ? s + NS : (s >= NS ? s - NS : s);
+}
 
 // z-chunk length of one block of a z-marching kernel on a (bx, by) grid of plane tiles: enough chunks
 // that the grid covers at least 4 blocks per SM of the 148, each chunk at least 4R planes long (the

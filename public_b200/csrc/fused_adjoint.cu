@@ -12,6 +12,7 @@
 
 #include "cruna_internal.cuh"
 #include "fused_common.cuh"
+#include "ops_common.cuh"
 
 namespace cruna {
 
@@ -34,7 +35,7 @@ struct AdjArgs {
   const double *q0;
   double *acc;
   double *qnext;
-  const double *yr;    // YX: the y direction's terms of the five equations, from the line engine
+  const double *yd;    // YX: the y derivatives of p, qs1..qs5 and v qs5, from the line engine
 };
 
 // per-direction contribution in the reference's order (ns_rho_rhou_p.f90:317-370 / 386-440 / 456-509)
@@ -76,12 +77,14 @@ __device__ __forceinline__ void adj_dir(int d, double u1, double u2, double u3, 
 // plane fields: 0..4 qs1..qs5, 5 p - p_ref, 6 u, 7 v ; column fields: 0..4 qs1..qs5, 5 p - p_ref, 6 w.
 // T is the type of the shared-memory fields and of the derivatives (double, or float for the
 // FP32-stencil precision); the assembly and the RK update stay in double.
-// YX: without the y derivatives (compact schemes along y), starting from a.yr: no y halos, no v in the plane.
+// YX: with the y derivatives read from a.yd (compact schemes along y): no y halos, no v in the plane.
 template <typename T, int R, bool PER, bool YX = false>
 __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(const __grid_constant__ AdjArgs a) {
   constexpr int RY = YX ? 0 : R;
   constexpr int PW = TX + 2 * R, PH = TY + 2 * RY, PS = PW * PH;
   constexpr int NS = ring_slots(R);
+  // 32-bit point offsets in FP64 (1.36 -> 1.27 ms at 256^3); at the 168 registers of FP32 they spill (1.09 -> 1.29)
+  using Idx = std::conditional_t<sizeof(T) == 8, int, long long>;
   constexpr int NPF = YX ? 7 : 8, NRF = 7, RS = TX * TY;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *plane = reinterpret_cast<T *>(smem_raw);          // [NPF][PH][PW]
@@ -110,7 +113,7 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
     rp[5 * RS] = T(v8[7] - a.p_ref);
     rp[6 * RS] = T(v8[6] * (1.0 / v8[5]));
   };
-  auto load8 = [&](long long pt, double *v8) {
+  auto load8 = [&](Idx pt, double *v8) {
     v8[0] = S0[pt]; v8[1] = S1[pt]; v8[2] = S2[pt]; v8[3] = S3[pt]; v8[4] = S4[pt];
     v8[5] = Q0[pt]; v8[6] = Q3[pt]; v8[7] = Q4[pt];
   };
@@ -118,7 +121,7 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
     const int gk = gidx(oz, kk);
     if (gk < 0 || !col) continue;
     double v8[8];
-    load8(colpt + (long long)n12 * gk, v8);
+    load8(colpt + Idx(n12) * gk, v8);
     put_ring(kk, v8);
   }
   // register prefetch of the ring plane k+R+1 and the centre (rho, rho*u, rho*v) of plane k+1
@@ -128,9 +131,9 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
   auto prefetch = [&](int kk, int kc) {
     const int gk = gidx(oz, kk);
     pf_ok = (gk >= 0 && col);
-    if (pf_ok) load8(colpt + (long long)n12 * gk, pf);
+    if (pf_ok) load8(colpt + Idx(n12) * gk, pf);
     if (col && kc < k1) {
-      const long long pt = colpt + (long long)n12 * kc;
+      const Idx pt = colpt + Idx(n12) * kc;
       pc[0] = Q0[pt];
       pc[1] = Q1[pt];
       pc[2] = Q2[pt];
@@ -141,11 +144,11 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
   constexpr int NHT = HaloSet<R, RY>::PER_THREAD;
   double hv[NHT][9];      // qs1..qs5, rho, rho*u, rho*v, p of the halo cells, one plane ahead
   auto halo_fetch = [&](int kk) {
-    const long long kofs = (long long)n12 * kk;
+    const Idx kofs = Idx(n12) * kk;
 #pragma unroll
     for (int h = 0; h < NHT; ++h) {
       if (hs.goff[h] < 0) continue;
-      const long long pt = hs.goff[h] + kofs;
+      const Idx pt = hs.goff[h] + kofs;
       hv[h][0] = S0[pt]; hv[h][1] = S1[pt]; hv[h][2] = S2[pt]; hv[h][3] = S3[pt]; hv[h][4] = S4[pt];
       hv[h][5] = Q0[pt]; hv[h][6] = Q1[pt]; hv[h][8] = Q4[pt];
       if constexpr (!YX) hv[h][7] = Q2[pt];
@@ -166,26 +169,26 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
       c[6 * PS] = T(u1);
       if constexpr (!YX) c[7 * PS] = T(u2);
     }
-    const long long kofs = (long long)n12 * k;
+    const Idx kofs = Idx(n12) * k;
     // epilogue inputs of this plane, issued before the barrier so their latency overlaps the stencils
-    const long long opt = (i0 + tx) + (long long)n1 * (j0 + ty) + kofs;
-    double e_y[5] = {0, 0, 0, 0, 0}, e_src[5] = {0, 0, 0, 0, 0}, e_q0[5] = {0, 0, 0, 0, 0}, e_acc[5] = {0, 0, 0, 0, 0};
+    const Idx opt = (i0 + tx) + n1 * (j0 + ty) + kofs;
+    double e_y[YX ? 7 : 1], e_src[5] = {0, 0, 0, 0, 0}, e_q0[5] = {0, 0, 0, 0, 0}, e_acc[5] = {0, 0, 0, 0, 0};
     if (inside) {
       if constexpr (YX) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) e_y[v] = a.yr[opt + v * N];
+        for (int v = 0; v < 7; ++v) e_y[v] = (a.yd + v * N)[opt];
       }
       if (a.src) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) e_src[v] = a.src[opt + v * N];
+        for (int v = 0; v < 5; ++v) e_src[v] = (a.src + v * N)[opt];
       }
       if (a.stage != 0) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) e_q0[v] = a.q0[opt + v * N];
+        for (int v = 0; v < 5; ++v) e_q0[v] = (a.q0 + v * N)[opt];
       }
       if (a.stage >= 2) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) e_acc[v] = a.acc[opt + v * N];
+        for (int v = 0; v < 5; ++v) e_acc[v] = (a.acc + v * N)[opt];
       }
     }
 #pragma unroll
@@ -207,12 +210,12 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
       const T *c = plane + (ty + RY) * PW + (tx + R);
       int so[NS];
 #pragma unroll
-      for (int m = -R; m <= R; ++m) so[m + R] = ((slot + m + NS) % NS) * NRF * RS + tid;
+      for (int m = -R; m <= R; ++m) so[m + R] = ring_slot<NS>(slot + m) * NRF * RS + tid;
       const double qs5 = c[4 * PS];
       const double gm1 = a.gamma - 1.0;
       const double u3 = ring[so[R] + 6 * RS];
       const double gpr = a.gamma * p_c / (rho_c * gm1);         // :293
-      double r1 = e_y[0], r2 = e_y[1], r3 = e_y[2], r4 = e_y[3], r5 = e_y[4];  // :296
+      double r1 = 0.0, r2 = 0.0, r3 = 0.0, r4 = 0.0, r5 = 0.0;  // :296
       {
         const double s = ox.scale;
         const double A = D1<T, R, PER>(ox, c, 1, i) * s, B = D1<T, R, PER>(ox, c + PS, 1, i) * s,
@@ -222,7 +225,9 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
         const double P = D1<T, R, PER>(ox, c + 5 * PS, 1, i) * s;
         adj_dir(0, u1, u2, u3, gpr, ir, qs5, a.gamma, A, B, Cc, D, E, Sx, P, r1, r2, r3, r4, r5);
       }
-      if constexpr (!YX) {
+      if constexpr (YX) {
+        adj_dir(1, u1, u2, u3, gpr, ir, qs5, a.gamma, e_y[1], e_y[2], e_y[3], e_y[4], e_y[5], e_y[6], e_y[0], r1, r2, r3, r4, r5);
+      } else {
         const double s = oy.scale;
         const double A = D1<T, R, PER>(oy, c, PW, j) * s, B = D1<T, R, PER>(oy, c + PS, PW, j) * s,
                      Cc = D1<T, R, PER>(oy, c + 2 * PS, PW, j) * s, D = D1<T, R, PER>(oy, c + 3 * PS, PW, j) * s,
@@ -258,23 +263,22 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
       const double kv[5] = {r1, r2, r3, r4, r5};
       if (a.stage == 0) {
 #pragma unroll
-        for (int v = 0; v < 5; ++v) a.rhs[opt + v * N] = kv[v];
+        for (int v = 0; v < 5; ++v) (a.rhs + v * N)[opt] = kv[v];
       } else {
         const double dt = a.dt, dth = a.dt * 0.5;
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
-          const long long o = opt + v * N;
           if (a.stage == 1) {
-            a.acc[o] = kv[v];
-            a.qnext[o] = e_q0[v] + dth * kv[v];
+            (a.acc + v * N)[opt] = kv[v];
+            (a.qnext + v * N)[opt] = e_q0[v] + dth * kv[v];
           } else if (a.stage == 2) {
-            a.acc[o] = e_acc[v] + 2.0 * kv[v];
-            a.qnext[o] = e_q0[v] + dth * kv[v];
+            (a.acc + v * N)[opt] = e_acc[v] + 2.0 * kv[v];
+            (a.qnext + v * N)[opt] = e_q0[v] + dth * kv[v];
           } else if (a.stage == 3) {
-            a.acc[o] = e_acc[v] + 2.0 * kv[v];
-            a.qnext[o] = e_q0[v] + dt * kv[v];
+            (a.acc + v * N)[opt] = e_acc[v] + 2.0 * kv[v];
+            (a.qnext + v * N)[opt] = e_q0[v] + dt * kv[v];
           } else {
-            a.qnext[o] = e_q0[v] + dt / 6.0 * (e_acc[v] + kv[v]);
+            (a.qnext + v * N)[opt] = e_q0[v] + dt / 6.0 * (e_acc[v] + kv[v]);
           }
         }
       }
@@ -764,8 +768,17 @@ void rhs_adjoint_fused(cruna_ctx *c, const double *qs_in, const double *q, const
   }
 }
 
-// adjoint RHS or RK stage with a compact scheme along y (march_y_supported): the y terms from the line
-// engine, x and z and the stage update in the z-marching pass.  380 bytes a point and stage against 560.
+// v = (rho v) / rho
+__global__ void k_adj_v(long long N, const double *__restrict__ q, double *__restrict__ v) {
+  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N; p += (long long)gridDim.x * blockDim.x)
+    v[p] = q[p + 2 * N] / q[p];
+}
+
+// adjoint RHS or RK stage with a compact scheme along y (march_y_supported): the y derivatives of qs1..qs5 and
+// v qs5 in one launch of the line engine, everything else in the z-marching pass.  v and the y derivative of the
+// frozen state's p are formed with the first stage of a step and stay in the workspace for the other three.
+// Mixing layer 256 x 192 x 128: the pass that also summed the y terms on the line engine took 600 us a stage,
+// the plain derivatives 240 (loop step 5.13 -> 3.56 ms).
 void rhs_adjoint_march_y(cruna_ctx *c, const double *qs_in, const double *q, const double *g, double *rhs, double *qsbc,
                          int stage, const double *qs0, double *acc, double *qnext, double dt) {
   const double *qs = qs_in;
@@ -774,7 +787,17 @@ void rhs_adjoint_march_y(cruna_ctx *c, const double *qs_in, const double *q, con
     bc_qs(c, qsbc, q, 0);
     qs = qsbc;
   }
-  dir_adjoint(c, 1, qs, q, c->tmp, true);
+  const long long N = c->g.N;
+  double *v = c->tmp, *yd = v + N;
+  if (stage <= 1) {
+    k_adj_v<<<(int)std::min<long long>((N + 255) / 256, 148LL * 32), 256, 0, c->stream>>>(N, q, v);
+    CRUNA_LAUNCH_CHECK(c);
+    apply_diff(c, 1, q + 4 * N, nullptr, yd, c->dx[1], 1);
+  }
+  FieldSet fs;
+  for (int f = 0; f < 5; ++f) fs.add(qs + f * N, nullptr, yd + (1 + f) * N);
+  fs.add(qs + 4 * N, v, yd + 6 * N);
+  apply_diff_set(c, 1, fs, c->dx[1]);
   bool walls = false;                                              // :518 without q: only the walls act
   for (const BCRow &b : c->bc) walls = walls || b.type == 100;
   AdjArgs a;
@@ -789,7 +812,7 @@ void rhs_adjoint_march_y(cruna_ctx *c, const double *qs_in, const double *q, con
   a.q0 = qs0;
   a.acc = acc;
   a.qnext = qnext;
-  a.yr = c->tmp;
+  a.yd = yd;
   a.stage = walls ? 0 : stage;
   a.rhs = a.stage == 0 ? rhs : nullptr;
   constexpr int R = 4;

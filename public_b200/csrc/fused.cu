@@ -647,8 +647,9 @@ void launch_passes(cruna_ctx *c, FusedArgs &a) {
                                             (int)smem_g_cl<T, R>()));
       cl_configured = true;
     }
-    static const int res_cl = resident_blocks(k_pass_g<T, R, PER, true>, TX * TY, smem_g_cl<T, R>());
-    a.kc = z_chunk_balanced(c->g.n3, bx * by, res_cl, sms, R, nz);
+    // two blocks an SM (registers and shared memory; the occupancy query does not report them for this kernel): 64^3
+    // runs 256 blocks of 8 planes in place of 128 of 16
+    a.kc = z_chunk_balanced(c->g.n3, bx * by, 2, sms, R, nz);
     ProfScope ps(c, "pass_g_closure");
     k_pass_g<T, R, PER, true><<<dim3(bx, by, nz), dim3(TX, TY), smem_g_cl<T, R>(), c->stream>>>(a);
     CRUNA_LAUNCH_CHECK(c);

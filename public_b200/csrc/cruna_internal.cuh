@@ -190,6 +190,12 @@ struct cruna_ctx {
   float *cl_x = nullptr, *cl_y = nullptr;  // features (12N) and outputs (6N), point-major
   double *diag = nullptr;          // diagnostics reduction scratch (partials + 2 results)
   bool snapshot_host = false;      // gradient snapshots in pinned host memory instead of HBM
+  struct PoolBuf {
+    void *p;
+    size_t bytes;
+    bool used;
+  };
+  std::vector<PoolBuf> pool;       // buffers of the gradient and objective calls (pool_take, capi.cu)
   std::vector<void *> snap_pinned;  // those host slots (one state each), kept for later gradient calls
   // step graphs (step_graph.cu): the cache of the current run call, or null outside one
   bool graphs_enabled = true;
@@ -276,6 +282,9 @@ class GraphScope {
 void graph_step(cruna_ctx *c, int kind, const void *a, const void *b, const void *d,
                 const std::function<void()> &body);
 double *dalloc(cruna_ctx *c, size_t count);
+void *pool_take(cruna_ctx *c, size_t bytes);
+void pool_give(cruna_ctx *c, void *p);
+void pool_trim(cruna_ctx *c, size_t keep);
 void ensure_generic(cruna_ctx *c);
 bool use_fused(const cruna_ctx *c);
 // learned closure (closure_mlp.cu, closure_ops.cu)

@@ -452,8 +452,7 @@ long long gradient_impl(cruna_ctx *c, const double *q0, int nsteps, int nsnap, c
   build_schedule(span, g.S, g.kbest, cost);
   const size_t bytes = sizeof(double) * (size_t)c->g.N * 5;
   auto alloc = [&](size_t b) {
-    void *p = nullptr;
-    CRUNA_CUDA_CHECK(cudaMalloc(&p, b));
+    void *p = pool_take(c, b);
     scratch.push_back(p);
     return static_cast<double *>(p);
   };
@@ -487,11 +486,11 @@ long long gradient_impl(cruna_ctx *c, const double *q0, int nsteps, int nsnap, c
   g.adjoint_step = adjoint_loop_step;
   if (g.discrete) g.qN = alloc(bytes);
   if (g.host_slots && span > 0) {  // optional, last: without room for it every restart crosses PCIe
-    void *p = nullptr;
-    if (cudaMalloc(&p, bytes) == cudaSuccess) {
+    try {
+      void *p = pool_take(c, bytes);
       scratch.push_back(p);
       g.enable_cache(static_cast<double *>(p));
-    } else {
+    } catch (const std::runtime_error &) {
       (void)cudaGetLastError();
     }
   }
@@ -516,8 +515,7 @@ double objective_direct_impl(cruna_ctx *c, const double *q0, int nsteps, const c
                              std::vector<void *> &scratch) {
   GraphScope graphs(c);
   auto alloc = [&](size_t b) {
-    void *p = nullptr;
-    CRUNA_CUDA_CHECK(cudaMalloc(&p, b));
+    void *p = pool_take(c, b);
     scratch.push_back(p);
     return static_cast<double *>(p);
   };

@@ -940,8 +940,7 @@ static void direct_loop_body(cruna_ctx *c, double *q, const int on[3]) {
     step_direct(c, q, q);
     if (c->has_q_bc) bc_q(c, q, 1);
     if (on[2]) halo(c, q, 5);
-    for (int d = 0; d < 3; ++d)
-      if (on[d]) apply_filter(c, d, q, c->st[5], 5);
+    apply_filters(c, on, q, c->st[5], 5);
   }
 }
 
@@ -957,8 +956,7 @@ static void adjoint_loop_body(cruna_ctx *c, double *qs, const double *q0, const 
     step_adjoint(c, qs, q0, g, qs);
     if (c->has_q_bc) bc_qs(c, qs, q0, 1);
     if (on[2]) halo(c, qs, 5);
-    for (int d = 0; d < 3; ++d)
-      if (on[d]) apply_filter(c, d, qs, c->st[5], 5);
+    apply_filters(c, on, qs, c->st[5], 5);
   }
 }
 

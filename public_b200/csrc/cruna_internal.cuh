@@ -213,6 +213,7 @@ void launch_line_solve(cruna_ctx *c, const LineOp &op, int dir, const double *in
 void apply_diff(cruna_ctx *c, int dir, const double *f1, const double *f2, double *out, double h,
                 int nfields);
 void apply_filter(cruna_ctx *c, int dir, double *q, double *scratch, int nfields);
+void apply_filters(cruna_ctx *c, const int on[3], double *q, double *scratch, int nfields);
 
 // RHS / BC / RK (ops.cu, fused.cu)
 // bc_mask: 1 applies the BC on q before, 2 the BC on the RHS after (3 = the reference order)

@@ -392,19 +392,36 @@ void apply_diff(cruna_ctx *c, int dir, const double *f1, const double *f2, doubl
   if (op.kind == OP_STENCIL && op.solve) launch_line_solve(c, op, dir, out, out, nfields);
 }
 
-// filter_i_d in place: compact filters on the line engine, which works in place; the others out of place
-// into scratch, solve, copy back
-void apply_filter(cruna_ctx *c, int dir, double *q, double *scratch, int nfields) {
+// filter_i_d of `in` into `out` (another buffer)
+static void filter_into(cruna_ctx *c, int dir, const double *in, double *out, int nfields) {
   const LineOp &op = c->fop[dir];
-  if (op.kind == OP_COPY) return;
   if (compact_fast(c, op)) {
-    for_sets(c, q, nullptr, q, nfields, [&](const FieldSet &fs) { launch_compact_set(c, op, dir, fs, 1.0); });
+    for_sets(c, in, nullptr, out, nfields, [&](const FieldSet &fs) { launch_compact_set(c, op, dir, fs, 1.0); });
     return;
   }
-  launch_line_stencil(c, op, dir, q, nullptr, scratch, 1.0, nfields);
-  if (op.solve) launch_line_solve(c, op, dir, scratch, scratch, nfields);
-  CRUNA_CUDA_CHECK(cudaMemcpyAsync(q, scratch, sizeof(double) * c->g.N * nfields,
-                                   cudaMemcpyDeviceToDevice, c->stream));
+  launch_line_stencil(c, op, dir, in, nullptr, out, 1.0, nfields);
+  if (op.solve) launch_line_solve(c, op, dir, out, out, nfields);
+}
+
+// the filters on[d] of i1, i2, i3 in turn, q in place: compact filters work in place on the line engine, the
+// others go to the other of q and scratch, and only an odd number of those ends with a copy back
+void apply_filters(cruna_ctx *c, const int on[3], double *q, double *scratch, int nfields) {
+  double *cur = q, *other = scratch;
+  for (int d = 0; d < 3; ++d) {
+    if (!on[d] || c->fop[d].kind == OP_COPY) continue;
+    if (compact_fast(c, c->fop[d])) {
+      filter_into(c, d, cur, cur, nfields);
+    } else {
+      filter_into(c, d, cur, other, nfields);
+      std::swap(cur, other);
+    }
+  }
+  if (cur != q) copy_state(c, q, cur, nfields);
+}
+
+void apply_filter(cruna_ctx *c, int dir, double *q, double *scratch, int nfields) {
+  const int on[3] = {dir == 0, dir == 1, dir == 2};
+  apply_filters(c, on, q, scratch, nfields);
 }
 
 // ------------------------------------------------------------------------------------------------

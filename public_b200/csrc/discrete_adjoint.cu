@@ -31,18 +31,15 @@ constexpr double kS1 = 110.4;  // Sutherland constant (ns_rho_rhou_p_trafos.f90:
 
 // backward workspace layout (fields of N points)
 enum VjpField {
-  V_L = 0,        // 5: D_d^T of the five RHS cotangents
-  V_MB = 5,       // 3: cotangent of rho u_d
-  V_UB = 8,       // 3: cotangent of u_v
-  V_PB = 11,      // 1: cotangent of p
-  V_TAUB = 12,    // 6: cotangents of tau_11, tau_22, tau_33, tau_12, tau_13, tau_23
-  V_MUB = 18,     // 1: cotangent of mu
-  V_TGB = 19,     // 3: cotangent of d_d T
-  V_GB = 22,      // 9: cotangent of d_d u_v, stored [d][v]
-  V_B = 31,       // 3: cotangent of d_v p
-  V_TB = 34,      // 1: cotangent of T
-  V_SCR = 35,     // 5: solve scratch of the transposed operators
-  kVjpFields = 40
+  V_MB = 0,       // 3: cotangent of rho u_d
+  V_UB = 3,       // 3: cotangent of u_v
+  V_PB = 6,       // 1: cotangent of p
+  V_TGB = 7,      // 3: cotangent of d_d T
+  V_GB = 10,      // 9: cotangent of d_d u_v, stored [d][v]
+  V_B = 19,       // 3: cotangent of d_v p
+  V_TB = 22,      // 1: cotangent of T
+  V_SCR = 23,     // 5: solve scratch of the transposed operators
+  kVjpFields = 28
 };
 
 // state-sized buffers (cruna_ctx::vjp_st)
@@ -549,74 +546,83 @@ void bc_rhs_T(cruna_ctx *c, const double *qb, double *lam, double *lam_q) {
 // ------------------------------------------------------------------------------------------------
 // transpose of the interior RHS (ns_rho_rhou_p.f90:95-209)
 // ------------------------------------------------------------------------------------------------
-// one direction's transposed derivatives of the five RHS components: mass (:131-135), momentum fluxes
-// and stress divergence (:138-177), pressure flux (:180-186), heat-flux divergence (:195-200)
-__global__ void k_vjp_dir(long long N, int d, double ratio, double gamma, double cp_pr, const double *__restrict__ q,
-                          const double *__restrict__ t, double *__restrict__ w) {
+// From the transposed derivatives L_d of the five RHS components along each live direction (workspace fields
+// l[d] .. l[d] + 4 of t): mass (:131-135), momentum fluxes and stress divergence (:138-177), pressure flux
+// (:180-186), heat-flux divergence (:195-200), then friction work and u . grad p (:187, :204-206), stresses (:118-128)
+// and Sutherland (trafos.f90:140).  One pass over memory: 72 field accesses a point, against 145 with one
+// accumulating kernel per direction (128 x 96 x 64, an RK stage: 260 us, now 108).
+struct VjpDirs {
+  int l[3];              // first L field, or -1 (empty direction)
+  double ratio[3];       // heat-flux spacing over flow spacing in D's scale
+};
+
+__global__ void k_vjp_point(long long N, const __grid_constant__ VjpDirs dirs, double gamma, double cp_pr,
+                            const double *__restrict__ q, const double *__restrict__ lam, const double *__restrict__ t,
+                            double *__restrict__ w) {
   const double gm1 = gamma - 1.0, gt = gamma / gm1;
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
        p += (long long)gridDim.x * blockDim.x) {
 #define W_(f) w[p + (long long)(f) * N]
 #define T_(f) t[p + (long long)(f) * N]
-    const double L0 = W_(V_L), L1 = W_(V_L + 1), L2 = W_(V_L + 2), L3 = W_(V_L + 3), L4 = W_(V_L + 4);
-    const double u0 = T_(F_U1), u1 = T_(F_U2), u2 = T_(F_U3);
-    const double md = q[p + (1 + d) * N], pr = q[p + 4 * N];
-    const double Lv[3] = {L1, L2, L3};
-    W_(V_MB + d) = W_(V_MB + d) - L0 - (u0 * L1 + u1 * L2 + u2 * L3);
-    for (int v = 0; v < 3; ++v) {
-      W_(V_UB + v) = W_(V_UB + v) - md * Lv[v];
-      W_(V_TAUB + tau_slot(v, d)) = W_(V_TAUB + tau_slot(v, d)) + Lv[v];
+    const double mu = T_(F_MU), T = T_(F_T), pr = q[p + 4 * N];
+    const double u[3] = {T_(F_U1), T_(F_U2), T_(F_U3)};
+    double ub[3] = {0.0, 0.0, 0.0}, tb[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, pb = 0.0, mub = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      double mb = 0.0, tgb = 0.0;
+      if (dirs.l[d] >= 0) {
+        const double L0 = T_(dirs.l[d]), L4 = T_(dirs.l[d] + 4);
+        const double Lv[3] = {T_(dirs.l[d] + 1), T_(dirs.l[d] + 2), T_(dirs.l[d] + 3)};
+        const double md = q[p + (1 + d) * N];
+        mb = -L0 - (u[0] * Lv[0] + u[1] * Lv[1] + u[2] * Lv[2]);
+#pragma unroll
+        for (int v = 0; v < 3; ++v) {
+          ub[v] = ub[v] - md * Lv[v];
+          tb[tau_slot(v, d)] = tb[tau_slot(v, d)] + Lv[v];
+        }
+        const double e = -gt * gm1 * L4;
+        ub[d] = ub[d] + pr * e;
+        pb = pb + u[d] * e;
+        const double hb = gm1 * dirs.ratio[d] * L4;
+        tgb = mu * cp_pr * hb;
+        mub = mub + cp_pr * T_(F_TX + d) * hb;
+      }
+      W_(V_MB + d) = mb;
+      W_(V_TGB + d) = tgb;
     }
-    const double e = -gt * gm1 * L4;
-    const double ud = d == 0 ? u0 : (d == 1 ? u1 : u2);
-    W_(V_UB + d) = W_(V_UB + d) + pr * e;
-    W_(V_PB) = W_(V_PB) + ud * e;
-    const double hb = gm1 * ratio * L4;
-    const double mu = T_(F_MU);
-    W_(V_TGB + d) = mu * cp_pr * hb;
-    W_(V_MUB) = W_(V_MUB) + cp_pr * T_(F_TX + d) * hb;
-#undef W_
-#undef T_
-  }
-}
-
-// friction work and u . grad p (:187, :204-206), stresses (:118-128), Sutherland (trafos.f90:140)
-__global__ void k_vjp_mid(long long N, double gamma, const double *__restrict__ lam, const double *__restrict__ t,
-                          double *__restrict__ w) {
-  const double gm1 = gamma - 1.0;
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N;
-       p += (long long)gridDim.x * blockDim.x) {
-#define W_(f) w[p + (long long)(f) * N]
-#define T_(f) t[p + (long long)(f) * N]
+    W_(V_PB) = pb;
     const double L5 = gm1 * lam[p + 4 * N];
     double G[3][3];
+#pragma unroll
     for (int v = 0; v < 3; ++v)
+#pragma unroll
       for (int d = 0; d < 3; ++d) G[v][d] = T_(F_UX + 3 * v + d);
     const double tau[6] = {T_(F_T11), T_(F_T22), T_(F_T33), T_(F_T12), T_(F_T13), T_(F_T23)};
-    const double mu = T_(F_MU), T = T_(F_T);
-    const double u[3] = {T_(F_U1), T_(F_U2), T_(F_U3)};
     const double P[3] = {T_(F_PX), T_(F_PY), T_(F_PZ)};
-    double tb[6];
-    for (int s = 0; s < 6; ++s) tb[s] = W_(V_TAUB + s);
     double Gb[3][3];
+#pragma unroll
     for (int v = 0; v < 3; ++v)
+#pragma unroll
       for (int d = 0; d < 3; ++d) {
         tb[tau_slot(v, d)] += L5 * G[v][d];
         Gb[v][d] = L5 * tau[tau_slot(v, d)];
       }
     const double div = G[0][0] + G[1][1] + G[2][2];
-    double mub = W_(V_MUB);
+#pragma unroll
     for (int v = 0; v < 3; ++v) mub += tb[v] * (-(2.0 / 3.0) * div + 2.0 * G[v][v]);
     mub += tb[3] * (G[0][1] + G[1][0]) + tb[4] * (G[0][2] + G[2][0]) + tb[5] * (G[1][2] + G[2][1]);
     const double st = tb[0] + tb[1] + tb[2];
+#pragma unroll
     for (int v = 0; v < 3; ++v)
-      for (int d = 0; d < 3; ++d)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
         Gb[v][d] += (v == d) ? 2.0 * mu * tb[v] - (2.0 / 3.0) * mu * st : mu * tb[tau_slot(v, d)];
-    for (int v = 0; v < 3; ++v)
-      for (int d = 0; d < 3; ++d) W_(V_GB + 3 * d + v) = Gb[v][d];
+        W_(V_GB + 3 * d + v) = Gb[v][d];
+      }
     W_(V_TB) = mub * mu * (1.5 / T - 1.0 / (T + kS1));
+#pragma unroll
     for (int v = 0; v < 3; ++v) {
-      W_(V_UB + v) = W_(V_UB + v) + L5 * P[v];
+      W_(V_UB + v) = ub[v] + L5 * P[v];
       W_(V_B + v) = -lam[p + (1 + v) * N] + L5 * u[v];
     }
 #undef W_
@@ -652,8 +658,6 @@ void interior_vjp(cruna_ctx *c, const double *qb, const double *lam, double *mu,
   generic_forward_gradients(c, qb);
   double *w = c->vjp_ws;
   auto Wf = [&](int f) { return w + (long long)f * N; };
-  CRUNA_CUDA_CHECK(cudaMemsetAsync(Wf(V_MB), 0, sizeof(double) * N * (V_MUB + 1 - V_MB), c->stream));
-  CRUNA_CUDA_CHECK(cudaMemsetAsync(Wf(V_TGB), 0, sizeof(double) * N * 3, c->stream));
   const int blocks = (int)std::min<long long>(nblocks(N), 148LL * 32);
   const double gamma = c->cfg.gamma;
   const double cp_pr = gamma * (c->cfg.R / c->cfg.W) / (gamma - 1.0) / c->cfg.Pr;
@@ -663,14 +667,19 @@ void interior_vjp(cruna_ctx *c, const double *qb, const double *lam, double *mu,
     live[d] = c->dop[d].kind != OP_ZERO;  // an empty direction contributes nothing (and has dx = inf)
     hT[d] = c->cfg.heat_flux_dx ? c->dx[d] : 1.0;
   }
+  // L_d in three runs of the workspace that the forward part leaves free (the flux terms beside grad p)
+  static const int slots[3] = {F_M1, F_V1X, F_V2X};
+  static_assert(F_M1 + 5 <= F_PX && F_V1X == F_PX + 1 && F_V1X + 5 <= F_PY && F_V2X == F_PY + 1 && F_V2X + 5 <= F_PZ,
+                "the L fields keep clear of grad p");
+  VjpDirs dirs;
   for (int d = 0; d < 3; ++d) {
+    dirs.l[d] = live[d] ? slots[d] : -1;
+    dirs.ratio[d] = 0.0;
     if (!live[d]) continue;
-    diff_T(c, d, lam, Wf(V_L), c->dx[d], 5, 0);
-    const double ratio = diff_scale(c, d, hT[d]) / diff_scale(c, d, c->dx[d]);
-    k_vjp_dir<<<blocks, kThreads, 0, c->stream>>>(N, d, ratio, gamma, cp_pr, qb, c->tmp, w);
-    CRUNA_LAUNCH_CHECK(c);
+    diff_T(c, d, lam, c->tmp + (long long)slots[d] * N, c->dx[d], 5, 0);
+    dirs.ratio[d] = diff_scale(c, d, hT[d]) / diff_scale(c, d, c->dx[d]);
   }
-  k_vjp_mid<<<blocks, kThreads, 0, c->stream>>>(N, gamma, lam, c->tmp, w);
+  k_vjp_point<<<blocks, kThreads, 0, c->stream>>>(N, dirs, gamma, cp_pr, qb, lam, c->tmp, w);
   CRUNA_LAUNCH_CHECK(c);
   for (int d = 0; d < 3; ++d) {
     if (!live[d]) continue;

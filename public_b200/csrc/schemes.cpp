@@ -112,8 +112,9 @@ bool build_line_table(int n, const std::vector<double> &dl, const std::vector<do
   for (int i = 0; i < n; ++i) {
     if (i > 0) l[i] = dl[i - 1] / u[i - 1];
     u[i] = i > 0 ? d[i] - l[i] * du[i - 1] : d[i];
-    // the schemes' matrices keep every pivot above 0.1 of their unit-size diagonal
-    if (!(std::fabs(u[i]) > 1e-3) || !(std::fabs(l[i]) < 1e2)) return false;
+    // the schemes' matrices and their transposes keep every pivot above 0.16 and every multiplier below 3.4 (filters
+    // with alpha <= 0.5 too); beyond that, elimination without interchanges would lose digits
+    if (!(std::fabs(u[i]) > 0.1) || !(std::fabs(l[i]) < 4.0)) return false;
     if (i < n - 1) c[i] = du[i] / u[i];
   }
   tab.assign((size_t)rows * 6, 0.0);

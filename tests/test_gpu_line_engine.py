@@ -45,6 +45,19 @@ def test_compact_operators_at_chunk_edges(length):
             assert np.max(np.abs(np.squeeze(got) - np.squeeze(ref))) < 1e-12 * np.max(np.abs(ref)), (scheme, d)
 
 
+@pytest.mark.parametrize("scheme", ["o6_i_c_p", "o10_i_c_o"])
+def test_filters_beyond_diagonal_dominance_keep_the_pivoted_solve(scheme):
+    # alpha > 0.5: elimination without row interchanges meets pivots of 0.02, so these take the general path
+    n = (40, 37, 33)
+    f = np.asfortranarray(np.random.default_rng(4).standard_normal(n))
+    kw = dict(n=n, diff=("empty",) * 3, filt=(scheme,) * 3, alpha=0.55)
+    with Cruna(Settings(**kw)) as c:
+        for d in range(3):
+            got = getattr(c, f"filter_i{d + 1}")(f)
+            ref = O.filter_dir(O.Config(**kw), d, f[..., None])[..., 0]
+            assert np.max(np.abs(np.squeeze(got) - ref)) < 1e-12 * np.max(np.abs(ref)), d
+
+
 MIXES = [("o6_i_c_p", "o6_i_c_p", "o6_i_c_p"), ("o6_i_c_o", "o4_i_c_p_pade", "o8_e_c_p"),
          ("o8_e_c_p", "o6_i_c_o", "o8_e_c_p"), ("o8_e_c_p", "o4_i_c_p_pade", "o8_e_c_p"),
          ("o4_e_c_o", "o4_i_c_o_pade", "empty"), ("o2_e_c_o", "o8_e_c_p", "o6_i_c_o"), ("empty", "empty", "o6_i_c_p")]

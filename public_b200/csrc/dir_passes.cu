@@ -6,9 +6,9 @@
 // u, v, w, T, rho u_d, rho u_d u_v, p, p u_d -- from the state, differentiates them with the whole line
 // resident in the block, writes the four gradients and adds the convective terms to five accumulators
 // (14 field accesses in place of 31); a pointwise pass turns gradients into stresses, heat fluxes and
-// friction work; one pass per direction adds the divergences of three stresses and the heat flux; the
-// last one finishes the RHS and makes the RK4 stage update.  Adjoint: one pass per direction differentiates
-// qs1..qs5, u_d qs5 and p and adds that direction's terms; the last one makes the stage update.
+// friction work; one pass per direction adds the divergences of three stresses and the heat flux; a pointwise
+// pass finishes the RHS and makes the RK4 stage update.  Adjoint: one pass per direction differentiates
+// qs1..qs5, u_d qs5 and p and adds that direction's terms; the same pass finishes.
 #include <algorithm>
 #include <cmath>
 
@@ -21,7 +21,7 @@ namespace {
 
 constexpr int L = kLineL;
 
-// what the last pass does with a finished RHS component (rk_o4_e.f90:45-50, :92-97)
+// what the last pass does with the finished RHS (rk_o4_e.f90:45-50, :92-97)
 struct Finish {
   int stage;            // 0: write rhs; 1..4: RK4 stage update
   double dt;

@@ -168,9 +168,11 @@ __global__ void __launch_bounds__(128) k_line_stencil_r(LineOp op, Grid g, const
 // Compact operators (explicit part, tridiagonal solve, cyclic correction) on the line engine, one field per
 // blockIdx.y; R = 0 solves the input itself.  Every load of a block precedes its first barrier and its stores
 // follow one, and a block owns whole lines, so out may be the input.  X: lines along x, staged through
-// shared memory with an odd row pitch (lanes on neighbouring lines then hit different banks).
+// shared memory with an odd row pitch (lanes on neighbouring lines then hit different banks).  Bound by the latency
+// of its window loads: four blocks an SM for radii up to 3 (six derivatives of 256 x 192 x 128 along y 190 -> 165 us),
+// three for the wider filters (four: 248 -> 263 us for five fields).
 template <int R, bool ANTI, bool X>
-__global__ void __launch_bounds__(kLineThreads, 3) k_lines(const __grid_constant__ LineOp op, Grid g, int dir,
+__global__ void __launch_bounds__(kLineThreads, R <= 3 ? 4 : 3) k_lines(const __grid_constant__ LineOp op, Grid g, int dir,
                                                   const __grid_constant__ FieldSet fs, double scale, int G, int C) {
   extern __shared__ double line_sm[];
   const LineBlock b = line_block<1>(op, line_sm, G, C);

@@ -6,6 +6,7 @@
 #include <string>
 
 #include "cruna_internal.cuh"
+#include "ops_common.cuh"
 
 using namespace cruna;
 
@@ -70,8 +71,10 @@ void pool_trim(cruna_ctx *c, size_t keep) {
   }
 }
 
+// the generic path's workspace: the passes on the line engine, the features and the discrete adjoint stay below
+// grad p's last field; only the sequence of single derivatives uses the rest
 void ensure_generic(cruna_ctx *c) {
-  if (!c->tmp) c->tmp = dalloc(c, (size_t)c->g.N * 60);
+  if (!c->tmp) c->tmp = dalloc(c, (size_t)c->g.N * (c->dir_ok ? F_PZ + 1 : kGenericFields));
 }
 
 bool use_fused(const cruna_ctx *c) { return c->fused_ok && !c->force_generic; }

@@ -134,6 +134,13 @@ T *upload(cruna_ctx *c, const std::vector<T> &v) {
 
 void attach_factors(cruna_ctx *c, LineOp &op, const HostFactors &hf) {
   if (!op.solve) return;
+  if (op.cyclic) op.fbrat = hf.fbrat;
+  std::vector<double> tab;
+  if (c->g.N < (1LL << 31) - 1 && build_line_table(op.n, hf.raw_dl, hf.raw_d, hf.raw_du,
+                                                   op.cyclic ? hf.fbnorm : std::vector<double>(), tab, op.kf, op.kb)) {
+    op.tab = upload(c, tab);  // the line engine serves the operator; the factors below are the general path's
+    return;
+  }
   std::vector<double> inv(hf.d.size());
   for (size_t i = 0; i < hf.d.size(); ++i) inv[i] = 1.0 / hf.d[i];
   op.dl = upload(c, hf.dl);
@@ -141,17 +148,7 @@ void attach_factors(cruna_ctx *c, LineOp &op, const HostFactors &hf) {
   op.du = upload(c, hf.du);
   op.du2 = upload(c, hf.du2);
   op.ipiv = upload(c, hf.ipiv);
-  op.nopiv = 1;
-  for (size_t i = 0; i + 1 < hf.ipiv.size(); ++i)
-    if (hf.ipiv[i] != (int)i + 1) op.nopiv = 0;
-  if (op.cyclic) {
-    op.fbnorm = upload(c, hf.fbnorm);
-    op.fbrat = hf.fbrat;
-  }
-  std::vector<double> tab;
-  if (build_line_table(op.n, hf.raw_dl, hf.raw_d, hf.raw_du, op.cyclic ? hf.fbnorm : std::vector<double>(), tab, op.kf,
-                       op.kb))
-    op.tab = upload(c, tab);
+  if (op.cyclic) op.fbnorm = upload(c, hf.fbnorm);
 }
 
 long long N5(const cruna_ctx *c) { return c->g.N * 5; }

@@ -71,8 +71,8 @@ void pool_trim(cruna_ctx *c, size_t keep) {
   }
 }
 
-// the generic path's workspace: the passes on the line engine, the features and the discrete adjoint stay below
-// grad p's last field; only the sequence of single derivatives uses the rest
+// the generic path's workspace: the direct RHS on the line engine's passes, the adjoint RHS, the features and the
+// discrete adjoint stay below grad p's last field; only the direct RHS as single derivatives uses the rest
 void ensure_generic(cruna_ctx *c) {
   if (!c->tmp) c->tmp = dalloc(c, (size_t)c->g.N * (c->dir_ok ? F_PZ + 1 : kGenericFields));
 }
@@ -224,7 +224,7 @@ void step_direct(cruna_ctx *c, const double *q0, double *q1) {
 
 // time_stepper_adjoint (rk_o4_e.f90:62-105): dt -> -dt, q0 frozen; qs1 may alias qs0
 void step_adjoint(cruna_ctx *c, const double *qs0, const double *q0, const double *g, double *qs1) {
-  double *k = ((use_fused(c) || c->dir_ok) && !c->has_rhs_bc) ? nullptr : rhs_buffer(c);
+  double *k = ((use_fused(c) || c->march_y_ok) && !c->has_rhs_bc) ? nullptr : rhs_buffer(c);
   double *acc = c->st[1], *qa = c->st[2], *qb = c->st[3], *qbc = c->st[4];
   const double dt = -c->cfg.dt;
   halo(c, q0, 5);

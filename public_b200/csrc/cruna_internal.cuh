@@ -137,7 +137,7 @@ struct cruna_ctx {
   std::string err;
   bool force_generic = false;
   bool fused_ok = false;
-  bool dir_ok = false;          // generic path on the per-direction passes (dir_passes.cu)
+  bool dir_ok = false;          // generic path: the direct RHS on the per-direction passes (dir_passes.cu)
   bool march_y_ok = false;      // generic path: x and z marching, y on the line engine (fused.cu)
   bool tma_fused = false;       // FP64 adjoint pass fed by TMA where the layout allows (cruna_set_tma_passes)
   bool filter_fused_ok = false;
@@ -220,18 +220,15 @@ void rhs_direct_generic(cruna_ctx *c, const double *q, double *rhs, double *qbc_
 void generic_forward_gradients(cruna_ctx *c, const double *q);  // primitives, grads, mu, tau into tmp
 void rhs_adjoint_generic(cruna_ctx *c, const double *qs, const double *q, const double *g, double *rhs,
                          double *qsbc_scratch);
-// the same RHS (stage 0) or RK stage on per-direction passes (dir_passes.cu), where they apply
+// the same direct RHS (stage 0) or RK stage on per-direction passes (dir_passes.cu), where they are the better path
 bool dir_passes_supported(const cruna_ctx *c);
 void rhs_direct_dir(cruna_ctx *c, const double *q, double *rhs, double *qbc_scratch, int bc_mask, int stage,
                     const double *q0, double *acc, double *qnext, double dt);
-void rhs_adjoint_dir(cruna_ctx *c, const double *qs, const double *q, const double *g, double *rhs,
-                     double *qsbc_scratch, int stage, const double *qs0, double *acc, double *qnext, double dt);
 bool only_sponge(const cruna_ctx *c);  // the RHS boundary table is one type-400 row
 // one direction's pass: gradients (slots F_UX + d, ...) and convective accumulators; stresses' and heat flux's
-// divergence onto r[1..4]; adjoint terms
+// divergence onto r[1..4]
 void dir_flux(cruna_ctx *c, int d, const double *q, double *t, double *r, bool first);
 void dir_viscous(cruna_ctx *c, int d, const double *t1, const double *t2, const double *t3, const double *h, double *r);
-void dir_adjoint(cruna_ctx *c, int d, const double *qs, const double *q, double *r, bool first);
 // x and z in the z-marching passes, y on the line engine (fused.cu, fused_adjoint.cu)
 bool march_y_supported(const cruna_ctx *c);
 void rhs_direct_march_y(cruna_ctx *c, const double *q, double *rhs, double *qbc_scratch, int bc_mask, int stage,

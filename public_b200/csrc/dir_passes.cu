@@ -1,14 +1,14 @@
-// RHS passes per direction for schemes with compact (tridiagonal) line operators, which the z-marching
-// passes do not take: right_hand_side_direct_3d and right_hand_side_adjoint_3d
-// (src/equations/ns_rho_rhou_p.f90:31-253, :257-536) as a few kernels on the line engine (lines.cuh).
+// Direct RHS passes per direction for schemes with compact (tridiagonal) line operators, which the z-marching
+// passes do not take: right_hand_side_direct_3d (src/equations/ns_rho_rhou_p.f90:31-253) as a few kernels on the
+// line engine (lines.cuh).
 //
-// Direct: one pass per direction d forms the ten quantities of :95-186 that are differentiated along d --
-// u, v, w, T, rho u_d, rho u_d u_v, p, p u_d -- from the state, differentiates them with the whole line
-// resident in the block, writes the four gradients and adds the convective terms to five accumulators
-// (14 field accesses in place of 31); a pointwise pass turns gradients into stresses, heat fluxes and
-// friction work; one pass per direction adds the divergences of three stresses and the heat flux; a pointwise
-// pass finishes the RHS and makes the RK4 stage update.  Adjoint: one pass per direction differentiates
-// qs1..qs5, u_d qs5 and p and adds that direction's terms; the same pass finishes.
+// One pass per direction d forms the ten quantities of :95-186 that are differentiated along d -- u, v, w, T,
+// rho u_d, rho u_d u_v, p, p u_d -- from the state, differentiates them with the whole line resident in the block,
+// writes the four gradients and adds the convective terms to five accumulators (14 field accesses in place of 31);
+// a pointwise pass turns gradients into stresses, heat fluxes and friction work; one pass per direction adds the
+// divergences of three stresses and the heat flux; a pointwise pass finishes the RHS and makes the RK4 stage update.
+// The adjoint RHS keeps its sequence of derivatives (rhs_adjoint_generic): the same kind of pass over its seven
+// quantities took 1.2 to 2 times as long as they do (5.9 against 4.5 ms an RK4 step on 256 x 128 x 128).
 #include <algorithm>
 #include <cmath>
 
@@ -25,17 +25,12 @@ constexpr int L = kLineL;
 struct Finish {
   int stage;            // 0: write rhs; 1..4: RK4 stage update
   double dt;
-  const double *add;    // forcing / adjoint source or null
+  const double *add;    // forcing or null
   double *rhs;
   const double *q0;
   double *acc, *qnext;
   const double *qref;   // type-400 sponge of the direct RHS: rhs -= shape (q - qref); null: none
   SpongeDev sponge;
-};
-
-// what the adjoint pass reads at a point before its stores
-struct AdjIn {
-  double m, al, be, o0, o1, r5;
 };
 
 struct DirArgs {
@@ -45,7 +40,7 @@ struct DirArgs {
   double scale, scale_h;       // 1 / (h div) of the flow's and of the heat flux's derivatives
   double WoR, gamma;
   int first;                   // the accumulators are written, not added to
-  const double *q, *qs;
+  const double *q;
   double *t;                   // gradients u_d, v_d, w_d, T_d (flux pass)
   const double *s[4];          // stresses tau_1d, tau_2d, tau_3d and the heat flux along d (viscous pass)
   double *r;                   // five accumulators
@@ -61,8 +56,9 @@ struct Quant {
 //   pre(p, at): what is read at p before the stores of kSub points' results (a store may alias the next point's read
 //               as far as the compiler knows, so reads and stores point by point would expose every latency)
 //   post(p, at, pre's value, d0, d1): takes the derivatives at p
-template <int R, bool SOLVE, bool X, bool IR, int kSub = 4>
+template <int R, bool SOLVE, bool X, bool IR>
 struct DirBlock {
+  static constexpr int kSub = 4;
   const DirArgs &a;
   LineBlock b;
   int base, s, line, nlines, l0, pitch;
@@ -339,62 +335,6 @@ __global__ void __launch_bounds__(kLineThreads, 2) k_dir_visc_div(const __grid_c
   }
 }
 
-// one direction's terms of the adjoint RHS (:304-370, :380-440, :450-509).  With X = u . D(qs2..qs4) +
-// gpr D qs5 + qs5 / rho D p they are: r1 += u_d X, r_{1+v} -= u_d D qs_{1+v}, r_{1+d} -= D qs1 + X,
-// r5 += -(g-1) D qs_{1+d} - g u_d D qs5 + (g-1) D(u_d qs5).  The last direction finishes.
-template <int R, bool SOLVE, bool X>
-__global__ void __launch_bounds__(kLineThreads, 2) k_dir_adj(const __grid_constant__ DirArgs a) {
-  extern __shared__ double dir_sm[];
-  DirBlock<R, SOLVE, X, true, X ? 4 : 2> B(a, dir_sm);   // (four points' reads spill along y and z)
-  const long long N = a.g.N;
-  const int d = a.dir;
-  const double *q = a.q, *qs = a.qs, *md = q + (1 + d) * N;
-  double *r = a.r;
-  const bool more = a.first == 0;
-  const double gamma = a.gamma, gm1 = gamma - 1.0;
-  // the sum X of every point, in the block's shared memory (32 registers a thread would spill)
-  double *xt = X ? B.tile + 3 * a.G * B.pitch : B.tile + (a.C * L + 3 * R + B.b.i0) * a.G + B.b.g;
-  const int xstep = X ? 1 : a.G;
-  auto xs = [&](int at) -> double & { return xt[at * xstep]; };
-#pragma unroll 1
-  for (int k = 0; k < 4; ++k) {
-    // k = 0: D qs2, D qs3; 1: D qs4, D p; 2: D qs5, D(u_d qs5); 3: D qs1.  X grows by al x + be y.
-    const double *f0 = qs + (k == 3 ? 0 : 2 * k + (k < 2 ? 1 : 0)) * N;
-    const double *f1 = k == 0 ? qs + 2 * N : (k == 1 ? q + 4 * N : qs + 4 * N);
-    const double *pa = k == 0 ? q + N : (k == 1 ? q + 3 * N : q + 4 * N), *pb = k == 0 ? q + 2 * N : qs + 4 * N;
-    const double fa = k == 3 ? 0.0 : (k == 2 ? gamma / gm1 : 1.0), fb = k < 2 ? 1.0 : 0.0;
-    double *o0 = r + (k == 3 ? 1 + d : (k == 2 ? 4 : 1 + 2 * k)) * N, *o1 = k == 0 ? r + 2 * N : r;
-    const bool two = k == 0 || k == 3, add0 = more || k >= 2;
-    const bool here = k == (d == 2 ? 1 : 0), second = d == 1;   // D qs_{1+d} comes in this batch, as its second quantity
-    double *r5 = r + 4 * N;
-    const Quant c0{f0, nullptr, false};
-    const Quant c1{k == 3 ? f0 : f1, k == 2 ? md : nullptr, false};
-    B.template run<AdjIn>(
-        c0, c1, a.scale, a.scale,
-        [=](int p, int) {
-          AdjIn i;
-          i.m = md[p];
-          i.al = fa * pa[p];
-          i.be = fb != 0.0 ? pb[p] : 0.0;
-          i.o0 = add0 ? o0[p] : 0.0;
-          i.o1 = two && more ? o1[p] : 0.0;
-          i.r5 = here && more ? r5[p] : 0.0;
-          return i;
-        },
-        [&](int p, int at, const AdjIn &i, double x, double y) {
-          const double ir = B.inv(at), ud = i.m * ir;
-          const double X_ = (k == 0 ? 0.0 : xs(at)) + ir * (i.al * x + i.be * y);  // k = 3: al = be = 0
-          xs(at) = X_;
-          if (k == 2) o0[p] = i.o0 - gamma * ud * x + gm1 * y;
-          else if (k == 3) o0[p] = i.o0 - x - X_;
-          else o0[p] = i.o0 - ud * x;
-          if (here) r5[p] = i.r5 - gm1 * (second ? y : x);
-          if (k == 0) o1[p] = i.o1 - ud * y;
-          else if (k == 3) o1[p] = i.o1 + ud * X_;
-        });
-  }
-}
-
 // the finished RHS from the accumulators (scale5 on the energy equation), forcing or source, the type-400
 // sponge, and the RK4 stage update
 __global__ void __launch_bounds__(256) k_dir_finish(const __grid_constant__ Finish f, Grid g, const double *__restrict__ q,
@@ -430,16 +370,16 @@ __global__ void __launch_bounds__(256) k_dir_finish(const __grid_constant__ Fini
   }
 }
 
-enum DirPass { PASS_FLUX, PASS_VISC, PASS_ADJ };
+enum DirPass { PASS_FLUX, PASS_VISC };
 
 template <int R, bool SOLVE, bool X>
 void launch_dir(cruna_ctx *c, DirPass pass, DirArgs &a) {
   a.C = line_chunks(a.op.n);
   a.G = line_group(a.C);
   const long long lines = a.g.N / a.op.n;
-  // tiles: two quantities (X), 1 / rho, the adjoint's sum
+  // tiles: two quantities (X), 1 / rho
   const size_t rows = X ? (size_t)(a.op.n | 1) : (size_t)a.C * L + 3 * R;
-  const size_t tiles = (X ? 2 : 0) + (pass == PASS_VISC ? 0 : 1) + (pass == PASS_ADJ ? 1 : 0);
+  const size_t tiles = (X ? 2 : 0) + (pass == PASS_VISC ? 0 : 1);
   const size_t sm = sizeof(double) * (line_smem_doubles(a.C, a.G, 2) + tiles * rows * a.G);
   auto go = [&](auto kernel) {
     if (sm > 48 * 1024)
@@ -447,8 +387,7 @@ void launch_dir(cruna_ctx *c, DirPass pass, DirArgs &a) {
     kernel<<<(unsigned)((lines + a.G - 1) / a.G), a.C * a.G, sm, c->stream>>>(a);
   };
   if (pass == PASS_FLUX) go(k_dir_flux<R, SOLVE, X>);
-  else if (pass == PASS_VISC) go(k_dir_visc_div<R, SOLVE, X>);
-  else go(k_dir_adj<R, SOLVE, X>);
+  else go(k_dir_visc_div<R, SOLVE, X>);
   CRUNA_LAUNCH_CHECK(c);
 }
 
@@ -461,9 +400,8 @@ void launch_dir_x(cruna_ctx *c, DirPass pass, DirArgs &a) {
 // compact schemes (radius 1 or 2) run the radius-2 kernels, explicit ones (1, 2 or 4) the radius-4 kernels:
 // coefficients past the scheme's radius are skipped
 void launch_dir_pass(cruna_ctx *c, DirPass pass, DirArgs &a) {
-  static const char *names[3][3] = {{"dir_flux_x", "dir_flux_y", "dir_flux_z"},
-                                    {"dir_visc_x", "dir_visc_y", "dir_visc_z"},
-                                    {"dir_adj_x", "dir_adj_y", "dir_adj_z"}};
+  static const char *names[2][3] = {{"dir_flux_x", "dir_flux_y", "dir_flux_z"},
+                                    {"dir_visc_x", "dir_visc_y", "dir_visc_z"}};
   ProfScope ps(c, names[pass][a.dir]);
   if (a.op.solve) launch_dir_x<2, true>(c, pass, a);
   else launch_dir_x<4, false>(c, pass, a);
@@ -519,7 +457,7 @@ bool only_sponge(const cruna_ctx *c) {   // the RHS boundary table is one type-4
 }
 
 // the passes of one direction, for rhs_direct_dir and for the z-marching passes that take their y
-// derivatives from here (fused.cu, fused_adjoint.cu)
+// derivatives from here (fused.cu)
 void dir_flux(cruna_ctx *c, int d, const double *q, double *t, double *r, bool first) {
   DirArgs a = dir_args(c, d);
   a.q = q;
@@ -537,15 +475,6 @@ void dir_viscous(cruna_ctx *c, int d, const double *t1, const double *t2, const 
   a.s[3] = h;
   a.r = r;
   launch_dir_pass(c, PASS_VISC, a);
-}
-
-void dir_adjoint(cruna_ctx *c, int d, const double *qs, const double *q, double *r, bool first) {
-  DirArgs a = dir_args(c, d);
-  a.qs = qs;
-  a.q = q;
-  a.r = r;
-  a.first = first;
-  launch_dir_pass(c, PASS_ADJ, a);
 }
 
 // every direction on the line engine: explicit operators of radius 1, 2 or 4, compact ones with a row table,
@@ -603,30 +532,6 @@ void rhs_direct_dir(cruna_ctx *c, const double *q_in, double *rhs, double *qbc, 
   if (split) {
     bc_rhs(c, rhs, q);                                    // :218
     if (stage) rk_stage(c, stage, dt, rhs, q0, acc, qnext);
-  }
-}
-
-// adjoint RHS (stage 0) or RK stage
-void rhs_adjoint_dir(cruna_ctx *c, const double *qs_in, const double *q, const double *g, double *rhs, double *qsbc,
-                     int stage, const double *qs0, double *acc, double *qnext, double dt) {
-  const double *qs = qs_in;
-  if (c->has_q_bc) {                                      // :287-290
-    copy_state(c, qsbc, qs_in, 5);
-    bc_qs(c, qsbc, q, 0);
-    qs = qsbc;
-  }
-  bool walls = false;                                     // :518 without q: only the walls act
-  for (const BCRow &b : c->bc) walls = walls || b.type == 100;
-  bool first = true;
-  for (int d = 0; d < 3; ++d) {
-    if (c->dop[d].kind == OP_ZERO) continue;
-    dir_adjoint(c, d, qs, q, c->tmp, first);
-    first = false;
-  }
-  finish(c, finish_args(c, walls ? 0 : stage, dt, g, rhs, qs0, acc, qnext), q, c->tmp, 1.0);
-  if (walls) {
-    bc_rhss(c, rhs, qs, nullptr);
-    if (stage) rk_stage(c, stage, dt, rhs, qs0, acc, qnext);
   }
 }
 

@@ -1104,10 +1104,6 @@ void stage_adjoint_generic(cruna_ctx *c, const double *qs, const double *q, cons
     rhs_adjoint_march_y(c, qs, q, g, k, qsbc, stage, qs0, acc, qnext, dt);
     return;
   }
-  if (c->dir_ok) {
-    rhs_adjoint_dir(c, qs, q, g, k, qsbc, stage, qs0, acc, qnext, dt);
-    return;
-  }
   rhs_adjoint_generic(c, qs, q, g, k, qsbc);
   rk_stage(c, stage, dt, k, qs0, acc, qnext);
 }
@@ -1116,10 +1112,6 @@ void rhs_adjoint_generic(cruna_ctx *c, const double *qs_in, const double *q, con
                          double *qsbc) {
   if (c->march_y_ok) {
     rhs_adjoint_march_y(c, qs_in, q, g, rhs, qsbc, 0, nullptr, nullptr, nullptr, 0.0);
-    return;
-  }
-  if (c->dir_ok) {
-    rhs_adjoint_dir(c, qs_in, q, g, rhs, qsbc, 0, nullptr, nullptr, nullptr, 0.0);
     return;
   }
   const long long N = c->g.N;

@@ -354,8 +354,11 @@ int cruna_optimize_dev(cruna_ctx *ctx, const double *q0, const cruna_objective *
    non-finite value is found in q (device pointer). */
 int cruna_check_state_dev(cruna_ctx *ctx, const double *q);
 
-/* Which RHS implementation the context uses: 1 = fused explicit kernels, 0 = generic line-operator
-   sequence (compact schemes, 204/200 boundary types).  force_generic=1 selects the generic one. */
+/* Which RHS implementation the context uses: 1 = fused explicit kernels, 0 = generic path (compact schemes,
+   204/200 boundary types).  force_generic=1 selects the generic one.  What it runs follows from the schemes and
+   sizes: a compact scheme along y between periodic o8 ones takes z-marching kernels with the y derivatives from the
+   line engine; other direct RHS with compact schemes take one pass per direction (explicit directions periodic o8), as
+   do periodic o8 grids of 2^20 points or more; everything else is a sequence of single derivatives. */
 int cruna_rhs_path(const cruna_ctx *ctx);
 int cruna_set_force_generic(cruna_ctx *ctx, int force_generic);
 /* FP64 fused adjoint pass: on = 1 feeds it by TMA (cp.async.bulk.tensor tiles, column boxes and RK

@@ -74,7 +74,7 @@ void pool_trim(cruna_ctx *c, size_t keep) {
 // the generic path's workspace: the direct RHS on the line engine's passes, the adjoint RHS, the features and the
 // discrete adjoint stay below grad p's last field; only the direct RHS as single derivatives uses the rest
 void ensure_generic(cruna_ctx *c) {
-  if (!c->tmp) c->tmp = dalloc(c, (size_t)c->g.N * (c->dir_ok ? F_PZ + 1 : kGenericFields));
+  if (!c->tmp) c->tmp = dalloc(c, (size_t)c->g.N * (c->dir_ok || c->march_y_ok ? F_PZ + 1 : kGenericFields));
 }
 
 bool use_fused(const cruna_ctx *c) { return c->fused_ok && !c->force_generic; }
@@ -189,7 +189,7 @@ double *rhs_buffer(cruna_ctx *c) {
 
 // time_stepper_direct (rk_o4_e.f90:17-58): q1 may alias q0
 void step_direct(cruna_ctx *c, const double *q0, double *q1) {
-  double *k = ((use_fused(c) || c->dir_ok) && !c->has_rhs_bc) ? nullptr : rhs_buffer(c);
+  double *k = ((use_fused(c) || c->dir_ok || c->march_y_ok) && !c->has_rhs_bc) ? nullptr : rhs_buffer(c);
   double *acc = c->st[1], *qa = c->st[2], *qb = c->st[3], *qbc = c->st[4];
   const double dt = c->cfg.dt;
   if (use_fused(c)) {

@@ -397,8 +397,8 @@ void launch_dir_x(cruna_ctx *c, DirPass pass, DirArgs &a) {
   else launch_dir<R, SOLVE, false>(c, pass, a);
 }
 
-// compact schemes (radius 1 or 2) run the radius-2 kernels, explicit ones (1, 2 or 4) the radius-4 kernels:
-// coefficients past the scheme's radius are skipped
+// compact schemes (radius 1 or 2) run the radius-2 kernels (coefficients past the radius are skipped), explicit
+// ones of radius 4 the radius-4 kernels
 void launch_dir_pass(cruna_ctx *c, DirPass pass, DirArgs &a) {
   static const char *names[2][3] = {{"dir_flux_x", "dir_flux_y", "dir_flux_z"},
                                     {"dir_visc_x", "dir_visc_y", "dir_visc_z"}};
@@ -477,19 +477,24 @@ void dir_viscous(cruna_ctx *c, int d, const double *t1, const double *t2, const 
   launch_dir_pass(c, PASS_VISC, a);
 }
 
-// every direction on the line engine: explicit operators of radius 1, 2 or 4, compact ones with a row table,
-// or empty ones, at least one direction live, lines of up to kLineMaxN points
+// The direct RHS on these passes where they are the better path: at least one compact direction (row table) or, on
+// grids of 2^20 points or more, none; explicit directions periodic o8.  RK4 steps in ms, passes against the
+// sequence of single derivatives (rhs_direct_generic): compact in every direction 128 x 120 x 96 periodic 2.48 / 2.80, 512^2 open
+// 0.99 / 1.37; o8 in every direction 256 x 128 x 128 6.40 / 6.83, but 1024 x 64 x 64 7.42 / 6.65 (a block holds few
+// long lines) and 32^3 0.74 / 0.67; explicit schemes of radius 1 and 2 run the radius-4 kernels and lose everywhere (open
+// o4 160^3 9.09 / 5.77, with a compact y 8.86 / 6.08).
 bool dir_passes_supported(const cruna_ctx *c) {
-  bool live = false;
   if (!line_grid_ok(c->g)) return false;
-  for (int d = 0; d < 3; ++d) {
-    const LineOp &op = c->dop[d];
+  bool compact = false, o8 = false;
+  for (const LineOp &op : c->dop) {
     if (op.kind == OP_ZERO) continue;
-    if (op.n > kLineMaxN) return false;
-    if (op.solve ? !(op.tab && op.r <= 2) : !(op.r == 1 || op.r == 2 || op.r == 4)) return false;
-    live = true;
+    if (op.solve ? !(op.tab && op.r <= 2) : op.r != 4) return false;
+    (op.solve ? compact : o8) = true;
   }
-  return live;
+  const int longest[3] = {compact ? 512 : 256, compact ? 1024 : 512, compact ? 1024 : 512};
+  for (int d = 0; d < 3; ++d)
+    if (c->dop[d].kind != OP_ZERO && !c->dop[d].solve && c->dop[d].n > longest[d]) return false;
+  return compact || (o8 && c->g.N >= 1LL << 20);
 }
 
 // direct RHS (stage 0) or RK stage of the state q_in; bc_mask as rhs_direct_generic

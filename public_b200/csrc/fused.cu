@@ -23,6 +23,7 @@
 
 #include "cruna_internal.cuh"
 #include "fused_common.cuh"
+#include "lines.cuh"
 #include "ops_common.cuh"
 
 namespace cruna {
@@ -832,7 +833,8 @@ bool march_y_supported(const cruna_ctx *c) {
     const LineOp &op = c->dop[d];
     if (op.kind != OP_STENCIL || op.solve || !op.periodic || op.r != 4) return false;
   }
-  return c->dir_ok && c->dop[1].kind == OP_STENCIL && c->dop[1].solve;
+  const LineOp &y = c->dop[1];
+  return line_grid_ok(c->g) && y.kind == OP_STENCIL && y.solve && y.tab && y.r <= 2;
 }
 
 void rhs_direct_march_y(cruna_ctx *c, const double *q_in, double *rhs, double *qbc, int bc_mask, int stage,

@@ -1,8 +1,9 @@
-"""Which kernels the generic path runs, by the names of the built-in profile: the sequence of single derivatives
-where it is the faster one, and that sequence against the oracle on lines that no other path takes."""
+"""Which kernels the generic path runs, by the names of the built-in profile, and the sequence of single
+derivatives against the oracle on lines that no other path takes."""
 import numpy as np
 import pytest
 
+from oracle import cruna_oracle as O
 from public_b200 import cases
 from public_b200.cruna import Cruna, Settings
 
@@ -30,3 +31,43 @@ def test_generic_adjoint_is_a_sequence_of_derivatives(diff):
     for d, scheme in zip("xyz", diff):
         assert ("compact_diff_" if "_i_" in scheme else "line_diff_") + d in names
     assert not any(k.startswith("dir_") for k in names)
+
+
+@pytest.mark.parametrize("diff, n, passes", [
+    (("o6_i_c_p",) * 3, (24, 20, 18), True), (("o6_i_c_o", "o8_e_c_p", "o6_i_c_p"), (24, 20, 18), True),
+    (("o8_e_c_p",) * 3, (128, 128, 64), True), (("o8_e_c_p",) * 3, (24, 20, 18), False),
+    (("o8_e_c_p",) * 3, (512, 64, 32), False), (("o4_e_c_o",) * 3, (24, 20, 18), False),
+    (("o4_e_c_p", "o6_i_c_o", "o4_e_c_p"), (24, 20, 18), False)])
+def test_generic_direct_passes_only_where_they_are_faster(diff, n, passes):
+    q = cases.smooth_random_state(n, seed=1)
+    with Cruna(Settings(n=n, diff=diff, **BASE)) as c:
+        c.force_generic(True)
+        names = kernels(c, lambda: c.time_stepper_direct(q))
+    assert ("dir_flux_x" in names) == passes
+    assert any(k.startswith(("line_diff_", "compact_diff_")) for k in names) != passes
+
+
+LONG = [(2049, 8, 9), (8, 2049, 8), (9, 8, 2049)]    # one line past the line engine: single derivatives throughout
+MIXED = [(33, 9, 18), (17, 16, 15)]                  # o8 along x or y beside compact directions: passes
+
+
+@pytest.mark.parametrize("n, diff", [(n, d) for n in LONG for d in (("o4_e_c_o", "o8_e_c_p", "o4_e_c_p"),
+                                                                    ("o6_i_c_p", "o6_i_c_o", "o4_i_c_p_pade"))]
+                         + [(n, d) for n in MIXED for d in (("o8_e_c_p", "o6_i_c_o", "o6_i_c_p"),
+                                                            ("o6_i_c_p", "o8_e_c_p", "o6_i_c_o"))])
+def test_rhs_and_steps_against_the_oracle(n, diff):
+    # RHS to 1e-12 relative L2 per variable plus 1e-13 max|q| / dx (one-sided closure rows), a step to dt times the latter
+    q = cases.smooth_random_state(n, seed=5)
+    rng = np.random.default_rng(7)
+    qs, g, f = (np.asfortranarray(0.1 * rng.standard_normal(q.shape)) for _ in range(3))
+    s = dict(BASE, n=n, diff=diff, dt=1e-6)  # dt within the viscous limit of 2049 points
+    S = O.Solver(O.Config(**s), force=f)
+    with Cruna(Settings(**s), force=f) as c:
+        c.force_generic(True)
+        floor = 1e-13 * np.max(np.abs(q)) / min(c.dx)
+        got = [(c.rhs_direct(q), S.rhs_direct(q), floor), (c.rhs_adjoint(qs, q, g), S.rhs_adjoint(qs, q, g), floor),
+               (c.time_stepper_direct(q), S.time_stepper_direct(q), s["dt"] * floor),
+               (c.time_stepper_adjoint(qs, q, g), S.time_stepper_adjoint(qs, q, g), s["dt"] * floor)]
+    for a, b, f0 in got:
+        for v in range(5):
+            assert np.linalg.norm(a[..., v] - b[..., v]) <= 1e-12 * np.linalg.norm(b[..., v]) + f0 * np.sqrt(b[..., v].size), v

@@ -132,25 +132,6 @@ T *upload(cruna_ctx *c, const std::vector<T> &v) {
   return static_cast<T *>(p);
 }
 
-void attach_factors(cruna_ctx *c, LineOp &op, const HostFactors &hf) {
-  if (!op.solve) return;
-  if (op.cyclic) op.fbrat = hf.fbrat;
-  std::vector<double> tab;
-  if (c->g.N < (1LL << 31) - 1 && build_line_table(op.n, hf.raw_dl, hf.raw_d, hf.raw_du,
-                                                   op.cyclic ? hf.fbnorm : std::vector<double>(), tab, op.kf, op.kb)) {
-    op.tab = upload(c, tab);  // the line engine serves the operator; the factors below are the general path's
-    return;
-  }
-  std::vector<double> inv(hf.d.size());
-  for (size_t i = 0; i < hf.d.size(); ++i) inv[i] = 1.0 / hf.d[i];
-  op.dl = upload(c, hf.dl);
-  op.inv_d = upload(c, inv);
-  op.du = upload(c, hf.du);
-  op.du2 = upload(c, hf.du2);
-  op.ipiv = upload(c, hf.ipiv);
-  if (op.cyclic) op.fbnorm = upload(c, hf.fbnorm);
-}
-
 long long N5(const cruna_ctx *c) { return c->g.N * 5; }
 
 double *stage_in(cruna_ctx *c, int slot, const double *host, int nfields) {
@@ -271,6 +252,32 @@ int dir_index(cruna_ctx *c, int dir) {
 }  // namespace
 
 namespace cruna {
+
+// the device side of a compact operator's solve: the line engine's row table where the matrix has one, the pivoted
+// factors otherwise
+void attach_factors(cruna_ctx *c, LineOp &op, const HostFactors &hf) {
+  if (!op.solve) return;
+  if (op.cyclic) op.fbrat = hf.fbrat;
+  op.tab = op.dl = op.inv_d = op.du = op.du2 = op.fbnorm = nullptr;
+  op.ipiv = nullptr;
+  std::vector<double> tab;
+  if (c->g.N < (1LL << 31) - 1 && build_line_table(op.n, hf.raw_dl, hf.raw_d, hf.raw_du,
+                                                   op.cyclic ? hf.fbnorm : std::vector<double>(), tab, op.kf, op.kb)) {
+    op.tab = upload(c, tab);
+    return;
+  }
+  std::vector<double> inv(hf.d.size());
+  for (size_t i = 0; i < hf.d.size(); ++i) inv[i] = 1.0 / hf.d[i];
+  op.dl = upload(c, hf.dl);
+  op.inv_d = upload(c, inv);
+  op.du = upload(c, hf.du);
+  op.du2 = upload(c, hf.du2);
+  op.ipiv = upload(c, hf.ipiv);
+  op.nopiv = 1;
+  for (size_t i = 0; i + 1 < hf.ipiv.size(); ++i)
+    if (hf.ipiv[i] != (int)i + 1) op.nopiv = 0;
+  if (op.cyclic) op.fbnorm = upload(c, hf.fbnorm);
+}
 
 int prof_begin(cruna_ctx *c, const char *name) {
   if (!c->prof_on) return -1;

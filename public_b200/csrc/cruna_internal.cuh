@@ -43,6 +43,7 @@ struct LineOp {
   double div = 1.0;                // explicit part is divided by (h * div): 12 for o4 explicit
   int solve = 0;                   // dgttrs follows
   int cyclic = 0;                  // Sherman-Morrison correction follows
+  int nopiv = 0;                   // dgttrf interchanged no rows (ipiv[i] == i + 1 throughout)
   double blend = 0.0;              // >0: out = q - blend * (q - F q)
   double fbrat = 0.0;
   // device factor arrays (owned by the context)
@@ -279,6 +280,7 @@ class GraphScope {
 void graph_step(cruna_ctx *c, int kind, const void *a, const void *b, const void *d,
                 const std::function<void()> &body);
 double *dalloc(cruna_ctx *c, size_t count);
+void attach_factors(cruna_ctx *c, LineOp &op, const HostFactors &hf);
 void *pool_take(cruna_ctx *c, size_t bytes);
 void pool_give(cruna_ctx *c, void *p);
 void pool_trim(cruna_ctx *c, size_t keep);

@@ -114,18 +114,12 @@ void build_transpose(cruna_ctx *c, const LineOp &op, const HostFactors &hf, Line
   ht.ipiv.assign(n, 0);
   if (lapack_dgttrf(n, ht.dl.data(), ht.d.data(), ht.du.data(), ht.du2.data(), ht.ipiv.data()) != 0)
     throw ApiError{CRUNA_ERR_UNSUPPORTED, "dgttrf of a transposed compact operator failed"};
-  std::vector<double> inv(ht.d.size());
-  for (size_t i = 0; i < ht.d.size(); ++i) inv[i] = 1.0 / ht.d[i];
+  ht.raw_dl = hf.raw_du;
+  ht.raw_d = hf.raw_d;
+  ht.raw_du = hf.raw_dl;
   t.sop = op;
   t.sop.cyclic = 0;
-  t.sop.tab = nullptr;
-  std::vector<double> tab;
-  if (build_line_table(n, hf.raw_du, hf.raw_d, hf.raw_dl, {}, tab, t.sop.kf, t.sop.kb)) t.sop.tab = upload_vec(c, tab);
-  t.sop.dl = upload_vec(c, ht.dl);
-  t.sop.inv_d = upload_vec(c, inv);
-  t.sop.du = upload_vec(c, ht.du);
-  t.sop.du2 = upload_vec(c, ht.du2);
-  t.sop.ipiv = upload_vec(c, ht.ipiv);
+  attach_factors(c, t.sop, ht);
 }
 
 __global__ void k_band_T(LineOpT op, Grid g, int dir, const double *__restrict__ in, double *__restrict__ out,

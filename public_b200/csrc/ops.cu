@@ -235,6 +235,169 @@ __global__ void __launch_bounds__(kLineThreads, R <= 3 ? 4 : 3) k_lines(const __
   }
 }
 
+// Compact operators along y or z, one thread per line, consecutive threads on consecutive x (every load and
+// store coalesced): dgttrs's sweeps with LAPACK's row interchanges, factors in shared memory.  EXPL: the explicit
+// part comes from a sliding window of f over the interior (one new load per point; the closure rows of open lines
+// use explicit_part) and the forward sweep runs on the fly, out of place; otherwise the line of `out` is solved in
+// place.  Then the backward sweep and the cyclic correction over the stored forward values.  Every sweep reads its
+// line CH points at a time and issues the next chunk's loads before it works through the current one.
+constexpr int kPerLineMaxN = 1024;  // factors in shared memory: 44 bytes per line point
+
+template <int R, bool ANTI, bool EXPL, bool NOPIV>
+__global__ void __launch_bounds__(64) k_line_compact_yz(LineOp op, Grid g, int dir,
+                                                        const double *__restrict__ f1,
+                                                        const double *__restrict__ f2, double *out,
+                                                        double scale, double sign, int nfields) {
+  constexpr int CH = 8;
+  constexpr int W = 2 * R + 1;
+  extern __shared__ double cs[];
+  const int n = op.n;
+  double *s_dl = cs, *s_du = cs + n, *s_du2 = cs + 2 * n, *s_inv = cs + 3 * n, *s_fb = cs + 4 * n;
+  int *s_piv = reinterpret_cast<int *>(cs + 5 * n);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    s_dl[i] = i < n - 1 ? op.dl[i] : 0.0;
+    s_du[i] = i < n - 1 ? op.du[i] : 0.0;
+    s_du2[i] = i < n - 2 ? op.du2[i] : 0.0;
+    s_inv[i] = op.inv_d[i];
+    s_fb[i] = op.cyclic ? op.fbnorm[i] : 0.0;
+    s_piv[i] = NOPIV ? i + 1 : op.ipiv[i];
+  }
+  __syncthreads();
+  const long long n12 = (long long)g.n1 * g.n2;
+  const long long nlines = g.N / n;
+  const long long total = nlines * nfields;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+       t += (long long)gridDim.x * blockDim.x) {
+    const long long fld = t / nlines, l = t - fld * nlines;
+    long long base, s;
+    if (dir == 1) { const long long i = l % g.n1, k = l / g.n1; base = i + k * n12; s = g.n1; }
+    else { base = l; s = n12; }
+    double *o = out + fld * g.N + base;
+    double *po = o;  // o[(i - 1) * s] for the forward step at i
+    double cur = 0.0;
+    // dgttrs forward sweep (L with LAPACK's row interchanges) on the pair (i - 1, i); v = b[i]
+    auto fwd = [&](int i, double v) {
+      if (i == 0) {
+        cur = v;
+        return;
+      }
+      if (NOPIV || s_piv[i - 1] == i) {
+        *po = cur;
+        cur = v - s_dl[i - 1] * cur;
+      } else {
+        *po = v;
+        cur = cur - s_dl[i - 1] * v;
+      }
+      po += s;
+    };
+    if (EXPL) {
+      const double *a = f1 + fld * g.N + base;
+      const double *b = f2 ? f2 + fld * g.N + base : nullptr;
+      const int ib = op.periodic ? 0 : op.nb, ie = op.periodic ? n : n - op.nb;
+      for (int i = 0; i < ib; ++i)
+        fwd(i, point_epilogue(op, explicit_part(op, a, b, 0, s, i), ldv(a, b, i * s), scale, sign));
+      auto wrap = [&](int idx) { return op.periodic ? (idx < 0 ? idx + n : (idx >= n ? idx - n : idx)) : idx; };
+      double w[W];  // w[R + m] = f(i + m)
+#pragma unroll
+      for (int m = 0; m < W; ++m) w[m] = ldv(a, b, wrap(ib + m - R) * s);
+      auto step = [&](int i, double next) {  // position i from the window, then slide it by one
+        const double v = interior_part<R, ANTI>(op, [&](int m) { return w[R + m]; });
+        fwd(i, point_epilogue(op, v, w[R], scale, sign));
+#pragma unroll
+        for (int m = 0; m < W - 1; ++m) w[m] = w[m + 1];
+        w[W - 1] = next;
+      };
+      // chunk at i0 needs f(i0 + u + 1 + R), u < CH, while i0 + u + 1 < ie
+      int i0 = ib;
+      double nx[CH];
+      if (i0 + CH <= ie) {
+#pragma unroll
+        for (int u = 0; u < CH; ++u) nx[u] = (i0 + u + 1 < ie) ? ldv(a, b, wrap(i0 + u + 1 + R) * s) : 0.0;
+      }
+      for (; i0 + CH <= ie; i0 += CH) {
+        double cb[CH];
+#pragma unroll
+        for (int u = 0; u < CH; ++u) cb[u] = nx[u];
+        if (i0 + 2 * CH <= ie) {
+#pragma unroll
+          for (int u = 0; u < CH; ++u)
+            nx[u] = (i0 + CH + u + 1 < ie) ? ldv(a, b, wrap(i0 + CH + u + 1 + R) * s) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < CH; ++u) step(i0 + u, cb[u]);
+      }
+      for (; i0 < ie; ++i0) step(i0, (i0 + 1 < ie) ? ldv(a, b, wrap(i0 + 1 + R) * s) : 0.0);
+      for (int i = ie; i < n; ++i)
+        fwd(i, point_epilogue(op, explicit_part(op, a, b, 0, s, i), ldv(a, b, i * s), scale, sign));
+    } else {
+      cur = o[0];
+      const double *pl = o + s;  // o[i0 * s]
+      int i0 = 1;
+      double nx[CH];
+      if (i0 + CH <= n) {
+#pragma unroll
+        for (int u = 0; u < CH; ++u) nx[u] = pl[(long long)u * s];
+      }
+      for (; i0 + CH <= n; i0 += CH) {
+        double cb[CH];
+#pragma unroll
+        for (int u = 0; u < CH; ++u) cb[u] = nx[u];
+        pl += CH * s;
+        if (i0 + 2 * CH <= n) {
+#pragma unroll
+          for (int u = 0; u < CH; ++u) nx[u] = pl[(long long)u * s];
+        }
+#pragma unroll
+        for (int u = 0; u < CH; ++u) fwd(i0 + u, cb[u]);
+      }
+      for (; i0 < n; ++i0, pl += s) fwd(i0, *pl);
+    }
+    // backward sweep with U (diagonal inverted, du, du2); po now points at o[(n - 1) * s]
+    double x2 = cur * s_inv[n - 1];
+    *po = x2;
+    const double xlast = x2;
+    double x1 = (po[-s] - s_du[n - 2] * x2) * s_inv[n - 2];  // n > 2R + 2 >= 4
+    po -= s;
+    *po = x1;
+    auto back = [&](int i, double bi) {
+      const double x0 = (bi - s_du[i] * x1 - s_du2[i] * x2) * s_inv[i];
+      po -= s;
+      *po = x0;
+      x2 = x1;
+      x1 = x0;
+    };
+    int i0 = n - 3;  // chunk at i0 reads positions i0 - u = po[-(u + 1) s]
+    double nb[CH];
+    if (i0 >= CH - 1) {
+#pragma unroll
+      for (int u = 0; u < CH; ++u) nb[u] = po[-(long long)(u + 1) * s];
+    }
+    for (; i0 >= CH - 1; i0 -= CH) {
+      double cb[CH];
+#pragma unroll
+      for (int u = 0; u < CH; ++u) cb[u] = nb[u];
+      if (i0 - CH >= CH - 1) {
+#pragma unroll
+        for (int u = 0; u < CH; ++u) nb[u] = po[-(long long)(CH + u + 1) * s];
+      }
+#pragma unroll
+      for (int u = 0; u < CH; ++u) back(i0 - u, cb[u]);
+    }
+    for (; i0 >= 0; --i0) back(i0, po[-s]);
+    if (op.cyclic) {  // Sherman-Morrison: x1 is the solution's first value, xlast its last
+      const double corr = x1 + op.fbrat * xlast;
+      for (int j0 = 0; j0 < n; j0 += CH) {
+        double bv[CH];
+#pragma unroll
+        for (int u = 0; u < CH; ++u) bv[u] = (j0 + u < n) ? o[(long long)(j0 + u) * s] : 0.0;
+#pragma unroll
+        for (int u = 0; u < CH; ++u)
+          if (j0 + u < n) o[(long long)(j0 + u) * s] = bv[u] - s_fb[j0 + u] * corr;
+      }
+    }
+  }
+}
+
 // the fast kernels handle interior radii 1..6 on lines longer than 2R + 2 (every periodic wrap then
 // stays within one period) whose open ends have at least R closure rows and an interior between them
 // (interior taps stay on the line)
@@ -291,6 +454,20 @@ static void launch_lines(cruna_ctx *c, const LineOp &op, int dir, const FieldSet
   CRUNA_LAUNCH_CHECK(c);
 }
 
+static size_t per_line_smem(const LineOp &op) { return (size_t)op.n * (5 * sizeof(double) + sizeof(int)); }
+
+template <int R, bool ANTI, bool EXPL>
+static void launch_per_line(cruna_ctx *c, const LineOp &op, int dir, const double *f1, const double *f2, double *out,
+                            double scale, int nfields) {
+  const int blocks = nblocks((c->g.N / op.n) * nfields, 64);  // small blocks spread few lines over all SMs
+  const size_t sm = per_line_smem(op);
+  if (op.nopiv)
+    k_line_compact_yz<R, ANTI, EXPL, true><<<blocks, 64, sm, c->stream>>>(op, c->g, dir, f1, f2, out, scale, 1.0, nfields);
+  else
+    k_line_compact_yz<R, ANTI, EXPL, false><<<blocks, 64, sm, c->stream>>>(op, c->g, dir, f1, f2, out, scale, 1.0, nfields);
+  CRUNA_LAUNCH_CHECK(c);
+}
+
 // contiguous fields f1 + k N (f2 + k N), out + k N, k < nfields, as field sets of at most kMax
 template <class F>
 static void for_sets(const cruna_ctx *c, const double *f1, const double *f2, double *out, int nfields, F &&fn) {
@@ -306,10 +483,24 @@ static const char *const kStencilNames[2][3] = {{"line_filter_x", "line_filter_y
                                                 {"line_diff_x", "line_diff_y", "line_diff_z"}};
 
 static bool stencil_fast(const cruna_ctx *c, const LineOp &op) { return fast_ok(op) && c->g.n2 <= 65535; }
-// compact operators on the line engine: every scheme of the tables above (derivatives of radius 1 and 2, filters
-// of radius 1 to 5) up to kLineMaxN points a line
-static bool compact_fast(const cruna_ctx *c, const LineOp &op) {
-  return line_grid_ok(c->g) && op.kind == OP_STENCIL && op.solve && op.tab && op.r <= (op.antisym ? 2 : 5);
+
+// How a compact operator runs on nfields fields: on the line engine (its row table); one thread per line with the
+// pivoted factors in shared memory (y and z, matrices without a table: filters with alpha > 0.5; five fields of
+// 128 x 512 x 96 along y, o6 filter: 0.35 ms against 0.99 as stencil and k_line_solve); or as these two.
+enum LineRoute { ROUTE_ENGINE, ROUTE_PER_LINE, ROUTE_GENERAL };
+
+static LineRoute line_route(const cruna_ctx *c, const LineOp &op, int dir, int nfields) {
+  (void)nfields;
+  if (op.tab && line_grid_ok(c->g)) return ROUTE_ENGINE;
+  return op.dl && dir > 0 && op.n >= 4 && op.n <= kPerLineMaxN ? ROUTE_PER_LINE : ROUTE_GENERAL;
+}
+
+// the route of the explicit part and the solve together: the engine and the per-line kernel take every scheme of
+// the tables above (derivatives of radius 1 and 2, filters of radius 1 to 5)
+static LineRoute compact_route(const cruna_ctx *c, const LineOp &op, int dir, int nfields) {
+  if (op.kind != OP_STENCIL || !op.solve || op.r > (op.antisym ? 2 : 5)) return ROUTE_GENERAL;
+  const LineRoute r = line_route(c, op, dir, nfields);
+  return r == ROUTE_PER_LINE && !fast_ok(op) ? ROUTE_GENERAL : r;
 }
 
 static void launch_stencil_set(cruna_ctx *c, const LineOp &op, int dir, const FieldSet &fs, double scale,
@@ -336,21 +527,27 @@ void launch_line_stencil(cruna_ctx *c, const LineOp &op, int dir, const double *
 void launch_line_solve(cruna_ctx *c, const LineOp &op, int dir, const double *in, double *out, int nfields) {
   static const char *names[3] = {"line_solve_x", "line_solve_y", "line_solve_z"};
   ProfScope ps(c, names[dir]);
-  if (op.tab && line_grid_ok(c->g)) {
+  const LineRoute route = line_route(c, op, dir, nfields);
+  if (route == ROUTE_ENGINE) {
     for_sets(c, in, nullptr, out, nfields, [&](const FieldSet &fs) { launch_lines<0, false>(c, op, dir, fs, 1.0); });
     return;
   }
-  const long long lines = (c->g.N / op.n) * nfields;
   copy_state(c, out, in, nfields);
+  if (route == ROUTE_PER_LINE) {
+    launch_per_line<1, false, false>(c, op, dir, nullptr, nullptr, out, 1.0, nfields);
+    return;
+  }
+  const long long lines = (c->g.N / op.n) * nfields;
   k_line_solve<<<nblocks(lines, 128), 128, 0, c->stream>>>(op, c->g, dir, out, nfields);
   CRUNA_LAUNCH_CHECK(c);
 }
 
-// explicit part and compact solve of op (compact_fast(op)) of every field of a set in one launch
-static void launch_compact_set(cruna_ctx *c, const LineOp &op, int dir, const FieldSet &fs, double scale) {
-  static const char *names[2][3] = {{"compact_filter_x", "compact_filter_y", "compact_filter_z"},
-                                    {"compact_diff_x", "compact_diff_y", "compact_diff_z"}};
-  ProfScope ps(c, names[op.antisym ? 1 : 0][dir]);
+static const char *const kCompactNames[2][3] = {{"compact_filter_x", "compact_filter_y", "compact_filter_z"},
+                                                {"compact_diff_x", "compact_diff_y", "compact_diff_z"}};
+
+// explicit part and compact solve of every field of a set in one launch of the line engine
+static void launch_engine_set(cruna_ctx *c, const LineOp &op, int dir, const FieldSet &fs, double scale) {
+  ProfScope ps(c, kCompactNames[op.antisym ? 1 : 0][dir]);
   if (op.antisym) {
     if (op.r == 1) launch_lines<1, true>(c, op, dir, fs, scale);
     else launch_lines<2, true>(c, op, dir, fs, scale);
@@ -365,6 +562,28 @@ static void launch_compact_set(cruna_ctx *c, const LineOp &op, int dir, const Fi
   }
 }
 
+// the same on nfields contiguous fields by the route that line_route chose (not the general one)
+static void launch_compact(cruna_ctx *c, LineRoute route, const LineOp &op, int dir, const double *f1, const double *f2,
+                           double *out, double scale, int nfields) {
+  if (route == ROUTE_ENGINE) {
+    for_sets(c, f1, f2, out, nfields, [&](const FieldSet &fs) { launch_engine_set(c, op, dir, fs, scale); });
+    return;
+  }
+  ProfScope ps(c, kCompactNames[op.antisym ? 1 : 0][dir]);
+  if (op.antisym) {
+    if (op.r == 1) launch_per_line<1, true, true>(c, op, dir, f1, f2, out, scale, nfields);
+    else launch_per_line<2, true, true>(c, op, dir, f1, f2, out, scale, nfields);
+    return;
+  }
+  switch (op.r) {
+    case 1: launch_per_line<1, false, true>(c, op, dir, f1, f2, out, scale, nfields); break;
+    case 2: launch_per_line<2, false, true>(c, op, dir, f1, f2, out, scale, nfields); break;
+    case 3: launch_per_line<3, false, true>(c, op, dir, f1, f2, out, scale, nfields); break;
+    case 4: launch_per_line<4, false, true>(c, op, dir, f1, f2, out, scale, nfields); break;
+    default: launch_per_line<5, false, true>(c, op, dir, f1, f2, out, scale, nfields); break;
+  }
+}
+
 // Dx_d of each field of a set (f1, or f1*f2 when every f2 is given), all with the same spacing h, in one
 // launch; the fallbacks take one apply_diff per field
 void apply_diff_set(cruna_ctx *c, int dir, const FieldSet &fs, double h) {
@@ -372,8 +591,8 @@ void apply_diff_set(cruna_ctx *c, int dir, const FieldSet &fs, double h) {
   const double scale = 1.0 / (h * op.div);
   bool uniform = true;
   for (int k = 1; k < fs.n; ++k) uniform = uniform && ((fs.f2[k] != nullptr) == (fs.f2[0] != nullptr));
-  if (compact_fast(c, op)) {
-    launch_compact_set(c, op, dir, fs, scale);
+  if (compact_route(c, op, dir, 1) == ROUTE_ENGINE) {
+    launch_engine_set(c, op, dir, fs, scale);
   } else if (uniform && !op.solve && stencil_fast(c, op)) {
     launch_stencil_set(c, op, dir, fs, scale, 1.0);
   } else {
@@ -381,24 +600,25 @@ void apply_diff_set(cruna_ctx *c, int dir, const FieldSet &fs, double h) {
   }
 }
 
-// Dx_d of f1 (or of f1*f2): explicit part scaled by 1/(h*div), then the compact solve if any
+// Dx_d(f1) or Dx_d(f1*f2) on nfields contiguous fields; h <= 0 or NaN means 1
 void apply_diff(cruna_ctx *c, int dir, const double *f1, const double *f2, double *out, double h,
                 int nfields) {
   const LineOp &op = c->dop[dir];
   const double scale = 1.0 / (h * op.div);
-  if (compact_fast(c, op)) {
-    for_sets(c, f1, f2, out, nfields, [&](const FieldSet &fs) { launch_compact_set(c, op, dir, fs, scale); });
+  const LineRoute route = compact_route(c, op, dir, nfields);
+  if (route != ROUTE_GENERAL) {
+    launch_compact(c, route, op, dir, f1, f2, out, scale, nfields);
     return;
   }
   launch_line_stencil(c, op, dir, f1, f2, out, scale, nfields);
   if (op.kind == OP_STENCIL && op.solve) launch_line_solve(c, op, dir, out, out, nfields);
 }
 
-// filter_i_d of `in` into `out` (another buffer)
-static void filter_into(cruna_ctx *c, int dir, const double *in, double *out, int nfields) {
+// filter_i_d of `in` into `out` (another buffer, except on the engine)
+static void filter_into(cruna_ctx *c, LineRoute route, int dir, const double *in, double *out, int nfields) {
   const LineOp &op = c->fop[dir];
-  if (compact_fast(c, op)) {
-    for_sets(c, in, nullptr, out, nfields, [&](const FieldSet &fs) { launch_compact_set(c, op, dir, fs, 1.0); });
+  if (route != ROUTE_GENERAL) {
+    launch_compact(c, route, op, dir, in, nullptr, out, 1.0, nfields);
     return;
   }
   launch_line_stencil(c, op, dir, in, nullptr, out, 1.0, nfields);
@@ -411,10 +631,11 @@ void apply_filters(cruna_ctx *c, const int on[3], double *q, double *scratch, in
   double *cur = q, *other = scratch;
   for (int d = 0; d < 3; ++d) {
     if (!on[d] || c->fop[d].kind == OP_COPY) continue;
-    if (compact_fast(c, c->fop[d])) {
-      filter_into(c, d, cur, cur, nfields);
+    const LineRoute route = compact_route(c, c->fop[d], d, nfields);
+    if (route == ROUTE_ENGINE) {
+      filter_into(c, route, d, cur, cur, nfields);
     } else {
-      filter_into(c, d, cur, other, nfields);
+      filter_into(c, route, d, cur, other, nfields);
       std::swap(cur, other);
     }
   }

@@ -71,3 +71,31 @@ def test_rhs_and_steps_against_the_oracle(n, diff):
     for a, b, f0 in got:
         for v in range(5):
             assert np.linalg.norm(a[..., v] - b[..., v]) <= 1e-12 * np.linalg.norm(b[..., v]) + f0 * np.sqrt(b[..., v].size), v
+
+
+@pytest.mark.parametrize("length", [24, 64, 1023, 1024, 1025])
+@pytest.mark.parametrize("scheme", ["o6_i_c_p", "o10_i_c_o"])
+def test_filters_beyond_diagonal_dominance_run_one_kernel_along_y_and_z(scheme, length):
+    # alpha > 0.5: no row table.  Both sides eliminate with row interchanges: 50 eps cond(B) of the field maximum
+    alpha = 0.55
+    B = np.eye(length) + alpha * (np.eye(length, k=1) + np.eye(length, k=-1))
+    if scheme.endswith("p"):
+        B[0, -1] = B[-1, 0] = alpha
+    else:
+        B[0, 1] = B[-1, -2] = 0.0
+    tol = 50 * np.finfo(float).eps * np.linalg.cond(B)
+    for d in (1, 2):
+        n = [3, 2, 2]
+        n[d] = length
+        n = tuple(n)
+        f = np.asfortranarray(np.random.default_rng(length).standard_normal(n))
+        filt = ["empty"] * 3
+        filt[d] = scheme
+        kw = dict(n=n, diff=("empty",) * 3, filt=tuple(filt), alpha=alpha)
+        out = []
+        with Cruna(Settings(**kw)) as c:
+            names = kernels(c, lambda: out.append(getattr(c, f"filter_i{d + 1}")(f)))
+        axis = "xyz"[d]
+        assert names == ({"compact_filter_" + axis} if length <= 1024 else {"line_filter_" + axis, "line_solve_" + axis})
+        ref = O.filter_dir(O.Config(**kw), d, f[..., None])[..., 0]
+        assert np.max(np.abs(np.squeeze(out[0]) - np.squeeze(ref))) <= tol * np.max(np.abs(ref)), d

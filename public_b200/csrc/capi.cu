@@ -253,8 +253,8 @@ int dir_index(cruna_ctx *c, int dir) {
 
 namespace cruna {
 
-// the device side of a compact operator's solve: the line engine's row table where the matrix has one, the pivoted
-// factors otherwise
+// the device side of a compact operator's solve: the line engine's row table where the matrix has one, and the
+// pivoted factors where another route may take the operator (line_route, ops.cu)
 void attach_factors(cruna_ctx *c, LineOp &op, const HostFactors &hf) {
   if (!op.solve) return;
   if (op.cyclic) op.fbrat = hf.fbrat;
@@ -264,7 +264,7 @@ void attach_factors(cruna_ctx *c, LineOp &op, const HostFactors &hf) {
   if (c->g.N < (1LL << 31) - 1 && build_line_table(op.n, hf.raw_dl, hf.raw_d, hf.raw_du,
                                                    op.cyclic ? hf.fbnorm : std::vector<double>(), tab, op.kf, op.kb)) {
     op.tab = upload(c, tab);
-    return;
+    if (op.n <= kLineEngineN) return;
   }
   std::vector<double> inv(hf.d.size());
   for (size_t i = 0; i < hf.d.size(); ++i) inv[i] = 1.0 / hf.d[i];

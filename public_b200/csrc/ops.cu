@@ -485,14 +485,29 @@ static const char *const kStencilNames[2][3] = {{"line_filter_x", "line_filter_y
 static bool stencil_fast(const cruna_ctx *c, const LineOp &op) { return fast_ok(op) && c->g.n2 <= 65535; }
 
 // How a compact operator runs on nfields fields: on the line engine (its row table); one thread per line with the
-// pivoted factors in shared memory (y and z, matrices without a table: filters with alpha > 0.5; five fields of
-// 128 x 512 x 96 along y, o6 filter: 0.35 ms against 0.99 as stencil and k_line_solve); or as these two.
+// pivoted factors in shared memory (y and z); or as a stencil and k_line_solve.  Matrices without a table (filters
+// with alpha > 0.5) take the second along y and z: five fields of 128 x 512 x 96 along y, o6 filter, 0.35 ms
+// against 0.99 with the third.
+// With a table, a launch of enough lines leaves the engine where its blocks hold few lines (line_group): four from
+// 385 points on, two from 769, one from 1537.  Along y and z a warp then uses 32 bytes of a sector or less, and one thread
+// per line, whose time hardly depends on the number of lines, is faster once they fill the SMs.  Five fields, lines a
+// field, o6 derivative, engine / per line in us (384 points, open, z, 16384 lines: 189 / 175):
+//   open      n = 448: 4096 lines 100 / 112, 8192 179 / 141;  n = 1024: 1024 lines 141 / 174, 2048 243 / 212, 8192 891 / 308
+//   periodic  (a sweep more) n = 640: 16384 lines 489 / 567;  n = 1024: 1024 lines 128 / 210, 4096 414 / 341, 8192 784 / 436
+// Along x past 1536 points one block an SM is left, and stencil and k_line_solve are faster on many lines:
+// n = 2048, 4096 lines, five fields: open 3047 / 2009, periodic 3102 / 2679; n = 1792: 2163 / 1992, 2262 / 2735.
 enum LineRoute { ROUTE_ENGINE, ROUTE_PER_LINE, ROUTE_GENERAL };
 
 static LineRoute line_route(const cruna_ctx *c, const LineOp &op, int dir, int nfields) {
-  (void)nfields;
-  if (op.tab && line_grid_ok(c->g)) return ROUTE_ENGINE;
-  return op.dl && dir > 0 && op.n >= 4 && op.n <= kPerLineMaxN ? ROUTE_PER_LINE : ROUTE_GENERAL;
+  const int n = op.n;
+  const long long lines = (c->g.N / n) * nfields;
+  const bool per_line = op.dl && dir > 0 && n >= 4 && n <= kPerLineMaxN;
+  if (op.tab && line_grid_ok(c->g)) {
+    const bool p = op.cyclic;
+    if (per_line && (n > 768 ? lines >= (p ? 16384 : 10240) : n > kLineEngineN && !p && lines >= 32768)) return ROUTE_PER_LINE;
+    return op.dl && dir == 0 && n > 1536 && lines >= (n > 1792 ? 12288 : (p ? 40960 : 20480)) ? ROUTE_GENERAL : ROUTE_ENGINE;
+  }
+  return per_line ? ROUTE_PER_LINE : ROUTE_GENERAL;
 }
 
 // the route of the explicit part and the solve together: the engine and the per-line kernel take every scheme of

@@ -99,3 +99,26 @@ def test_filters_beyond_diagonal_dominance_run_one_kernel_along_y_and_z(scheme, 
         assert names == ({"compact_filter_" + axis} if length <= 1024 else {"line_filter_" + axis, "line_solve_" + axis})
         ref = O.filter_dir(O.Config(**kw), d, f[..., None])[..., 0]
         assert np.max(np.abs(np.squeeze(out[0]) - np.squeeze(ref))) <= tol * np.max(np.abs(ref)), d
+
+
+@pytest.mark.parametrize("n, d, diff, filt", [
+    ((64, 400, 103), 1, "o6_i_c_o", "o10_i_c_o"), ((64, 32, 800), 2, "o6_i_c_o", "o6_i_c_o"),
+    ((64, 800, 52), 1, "o6_i_c_p", "o6_i_c_p"), ((64, 1024, 32), 1, "o4_i_c_o_pade", "o2_i_c_o"),
+    ((1800, 50, 50), 0, "o6_i_c_o", "o10_i_c_o")])
+def test_long_lines_leave_the_line_engine_on_many_lines(n, d, diff, filt):
+    # five fields at the sizes where the rule changes: to 1e-12 of the field maximum, as the operator parity tests
+    f = np.asfortranarray(np.random.default_rng(n[d]).standard_normal((*n, 5)))
+    dd, ff, x1 = ["empty"] * 3, ["empty"] * 3, [1.0] * 3
+    dd[d], ff[d] = diff, filt
+    kw = dict(n=n, diff=tuple(dd), filt=tuple(ff), x1=tuple(x1), alpha=0.45)
+    got = {}
+    with Cruna(Settings(**kw)) as c:
+        names = kernels(c, lambda: got.update(dx=getattr(c, f"Dx{d + 1}")(f, h=c.dx[d]), filt=getattr(c, f"filter_i{d + 1}")(f)))
+        h = c.dx[d]
+    assert ("line_solve_x" in names) == (d == 0)
+    cfg = O.Config(**kw)
+    for v in range(5):
+        ref = O.Dx(cfg, d, np.asfortranarray(f[..., v]), h)
+        assert np.max(np.abs(got["dx"][..., v] - ref)) < 1e-12 * np.max(np.abs(ref)), v
+    ref = O.filter_dir(cfg, d, f)
+    assert np.max(np.abs(got["filt"] - ref)) < 1e-12 * np.max(np.abs(ref))

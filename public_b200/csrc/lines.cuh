@@ -8,7 +8,8 @@
 // with the products of the sweep's multipliers (LU without row interchanges: y_i = v_i - l_i y_{i-1},
 // x_i = y_i / u_i - c_i x_{i+1}; a chunk's result depends on its incoming value y through Pf_i y).  The
 // incoming value is folded from the last kf chunk ends only: the multipliers decay, and the host picks kf so
-// that the part left out is below 1e-20 of a chunk end (all chunks where they do not decay).
+// that the part left out is below 1e-20 of a chunk end (all chunks where they do not decay).  A block that meets
+// an infinity or NaN folds every chunk, so that it reaches the whole line as in a sequential solve.
 #pragma once
 
 #include "ops_common.cuh"
@@ -57,6 +58,15 @@ __device__ __forceinline__ LineBlock line_block(const LineOp &op, double *smem, 
   return b;
 }
 
+// barrier; true where any thread's chunk ends x[q] hold an infinity or NaN
+template <int NB>
+__device__ __forceinline__ bool line_sync_nonfinite(const double (&x)[NB]) {
+  bool bad = false;
+#pragma unroll
+  for (int q = 0; q < NB; ++q) bad = bad || !isfinite(x[q]);
+  return __syncthreads_or(bad);
+}
+
 // solves B x = v for NB right-hand sides at once; every thread of the block calls it
 template <int NB>
 __device__ __forceinline__ void line_solve(const LineOp &op, const LineBlock &b, double (&v)[NB][kLineL]) {
@@ -67,13 +77,16 @@ __device__ __forceinline__ void line_solve(const LineOp &op, const LineBlock &b,
 #pragma unroll
     for (int q = 0; q < NB; ++q) v[q][k] = v[q][k] - l * v[q][k - 1];
   }
-#pragma unroll
-  for (int q = 0; q < NB; ++q) b.fwd[(q * b.C + b.c) * b.G + b.g] = v[q][kLineL - 1];
-  __syncthreads();
   double in[NB];
 #pragma unroll
+  for (int q = 0; q < NB; ++q) {
+    in[q] = v[q][kLineL - 1];
+    b.fwd[(q * b.C + b.c) * b.G + b.g] = in[q];
+  }
+  const int kf = line_sync_nonfinite<NB>(in) ? b.C : op.kf;
+#pragma unroll
   for (int q = 0; q < NB; ++q) in[q] = 0.0;
-  for (int j = max(0, b.c - op.kf); j < b.c; ++j) {
+  for (int j = max(0, b.c - kf); j < b.c; ++j) {
     const double pf = b.tab[3 * (j * kLineL + kLineL - 1)].y;
 #pragma unroll
     for (int q = 0; q < NB; ++q) in[q] = b.fwd[(q * b.C + j) * b.G + b.g] + pf * in[q];
@@ -89,11 +102,14 @@ __device__ __forceinline__ void line_solve(const LineOp &op, const LineBlock &b,
     }
   }
 #pragma unroll
-  for (int q = 0; q < NB; ++q) b.bwd[(q * b.C + b.c) * b.G + b.g] = v[q][0];
-  __syncthreads();
+  for (int q = 0; q < NB; ++q) {
+    in[q] = v[q][0];
+    b.bwd[(q * b.C + b.c) * b.G + b.g] = in[q];
+  }
+  const int kb = line_sync_nonfinite<NB>(in) ? b.C : op.kb;
 #pragma unroll
   for (int q = 0; q < NB; ++q) in[q] = 0.0;
-  for (int j = min(b.C - 1, b.c + op.kb); j > b.c; --j) {
+  for (int j = min(b.C - 1, b.c + kb); j > b.c; --j) {
     const double qb = b.tab[3 * (j * kLineL) + 2].x;
 #pragma unroll
     for (int q = 0; q < NB; ++q) in[q] = b.bwd[(q * b.C + j) * b.G + b.g] + qb * in[q];

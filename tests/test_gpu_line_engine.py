@@ -95,3 +95,30 @@ def test_sponge_in_the_last_pass_or_after_it(rows):
     with Cruna(Settings.from_dict(s), qref=q) as c:
         close(c.rhs_direct(qp), S.rhs_direct(qp))
         close(c.calc_direct(qp, 2), S.calc_direct(qp, 2))
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("at", [0, 47, 149])
+def test_a_non_finite_value_reaches_its_whole_line_and_no_other(at, bad):
+    # a sequential solve carries it to both ends; the lines beside it keep their values to rounding (1e-14 of the maximum)
+    rng = np.random.default_rng(3)
+    for d in range(3):
+        for diff, filt in (("o6_i_c_o", "o10_i_c_o"), ("o6_i_c_p", "o6_i_c_p")):
+            n = [6, 5, 7]
+            n[d] = 150
+            dd, ff, x1 = ["empty"] * 3, ["empty"] * 3, [1.0] * 3
+            dd[d], ff[d] = diff, filt
+            f = np.asfortranarray(rng.standard_normal(n))
+            g = f.copy(order="F")
+            where = [2, 3, 4]
+            where[d] = at
+            g[tuple(where)] = bad
+            with Cruna(Settings(n=tuple(n), diff=tuple(dd), filt=tuple(ff), x1=tuple(x1), alpha=0.45)) as c:
+                ops = [getattr(c, f"Dx{d + 1}"), getattr(c, f"filter_i{d + 1}")]
+                out = [(np.asarray(op(f)).reshape(n, order="F"), np.asarray(op(g)).reshape(n, order="F")) for op in ops]
+            line = tuple(slice(None) if k == d else where[k] for k in range(3))
+            for clean, got in out:
+                assert not np.any(np.isfinite(got[line])), (d, diff)
+                rest = np.ones(n, dtype=bool)
+                rest[line] = False
+                assert np.max(np.abs(got[rest] - clean[rest])) <= 1e-14 * np.max(np.abs(clean)), (d, diff)

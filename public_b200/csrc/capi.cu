@@ -1,7 +1,9 @@
 // extern "C" entry points of the CRUNA B200 library (declared in include/cruna_b200.h).
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 
@@ -12,51 +14,27 @@ using namespace cruna;
 
 namespace cruna {
 
-double *dalloc(cruna_ctx *c, size_t count) {
-  void *p = nullptr;
-  cudaError_t e = cudaMalloc(&p, count * sizeof(double));
-  if (e != cudaSuccess && !c->pool.empty()) {
-    cudaGetLastError();
-    pool_trim(c, 0);
-    e = cudaMalloc(&p, count * sizeof(double));
-  }
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    throw ApiError{CRUNA_ERR_NOMEM, std::string("cudaMalloc of ") + std::to_string(count * 8) +
-                                        " bytes failed: " + cudaGetErrorString(e)};
-  }
-  c->allocations.push_back(p);
-  return static_cast<double *>(p);
-}
-
 // Work buffers of the gradient, objective and optimisation calls.  A call takes its buffers here and gives them
-// back; up to kPoolMax bytes stay with the context for its next call (allocating and freeing six states of
-// 31 MB cost a 22 ms gradient call 4 to 20 ms), the rest is freed.  Every use is ordered on the context's stream.
+// back; the context keeps up to kPoolMax bytes of them for its next call (allocating and freeing six states of
+// 31 MB cost a 22 ms gradient call 4 to 20 ms), but after a call that allocated some no more than an eighth of the device
+// memory then free (asking costs 0.3 ms), and frees the rest.  Reuse is ordered on the context's stream; the copy stream of host snapshots is waited for before a
+// call gives its buffers back.  Every device allocation of the library goes through device_malloc, which frees what the
+// pools of all contexts on the device hold unused before it fails; other allocators of the process do not know the pools.
 constexpr size_t kPoolMax = size_t(1) << 30;
 
-void *pool_take(cruna_ctx *c, size_t bytes) {
-  for (auto &b : c->pool)
-    if (!b.used && b.bytes == bytes) {
-      b.used = true;
-      return b.p;
-    }
-  void *p = nullptr;
-  if (cudaMalloc(&p, bytes) != cudaSuccess) {  // room held for other sizes goes first
-    cudaGetLastError();
-    pool_trim(c, 0);
-    CRUNA_CUDA_CHECK(cudaMalloc(&p, bytes));
-  }
-  c->pool.push_back({p, bytes, true});
-  return p;
+namespace {
+
+struct PoolOwners {  // contexts with pool buffers; the mutex guards every pool
+  std::mutex m;
+  std::vector<cruna_ctx *> c;
+};
+PoolOwners &pool_owners() {
+  static PoolOwners *o = new PoolOwners;  // never destroyed: contexts may close after static destructors ran
+  return *o;
 }
 
-void pool_give(cruna_ctx *c, void *p) {
-  for (auto &b : c->pool)
-    if (b.p == p) b.used = false;
-  pool_trim(c, kPoolMax);
-}
-
-// frees unused buffers until at most `keep` bytes of them are left
+// frees unused buffers of c until at most `keep` bytes of them are left (the mutex is held).  cudaFree waits for
+// the device, so work in flight on a buffer is done before it goes.
 void pool_trim(cruna_ctx *c, size_t keep) {
   size_t held = 0;
   for (size_t i = 0; i < c->pool.size();) {
@@ -69,6 +47,77 @@ void pool_trim(cruna_ctx *c, size_t keep) {
     if (!b.used) held += b.bytes;
     ++i;
   }
+}
+
+}  // namespace
+
+cudaError_t device_malloc(void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  int dev = 0;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  {
+    std::lock_guard<std::mutex> lock(pool_owners().m);
+    for (cruna_ctx *c : pool_owners().c)
+      if (c->device == dev) pool_trim(c, 0);
+  }
+  return cudaMalloc(p, bytes);
+}
+
+double *dalloc(cruna_ctx *c, size_t count) {
+  void *p = nullptr;
+  const cudaError_t e = device_malloc(&p, count * sizeof(double));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    throw ApiError{CRUNA_ERR_NOMEM, std::string("cudaMalloc of ") + std::to_string(count * 8) +
+                                        " bytes failed: " + cudaGetErrorString(e)};
+  }
+  c->allocations.push_back(p);
+  return static_cast<double *>(p);
+}
+
+void *pool_take(cruna_ctx *c, size_t bytes) {
+  PoolOwners &o = pool_owners();
+  {
+    std::lock_guard<std::mutex> lock(o.m);
+    for (auto &b : c->pool)
+      if (!b.used && b.bytes == bytes) {
+        b.used = true;
+        return b.p;
+      }
+  }
+  void *p = nullptr;
+  CRUNA_CUDA_CHECK(device_malloc(&p, bytes));
+  std::lock_guard<std::mutex> lock(o.m);
+  if (std::find(o.c.begin(), o.c.end(), c) == o.c.end()) o.c.push_back(c);
+  c->pool.push_back({p, bytes, true});
+  c->pool_grown = true;
+  return p;
+}
+
+void pool_give(cruna_ctx *c, std::vector<void *> &bufs) {
+  size_t free_bytes = 0, total = 0;
+  if (c->pool_grown && cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+    cudaGetLastError();
+    free_bytes = 0;
+  }
+  std::lock_guard<std::mutex> lock(pool_owners().m);
+  for (void *p : bufs)
+    for (auto &b : c->pool)
+      if (b.p == p) b.used = false;
+  bufs.clear();
+  if (c->pool_grown) pool_trim(c, std::min(kPoolMax, free_bytes / 8));
+  c->pool_grown = false;
+}
+
+// a closing context's buffers
+static void pool_free(cruna_ctx *c) {
+  PoolOwners &o = pool_owners();
+  std::lock_guard<std::mutex> lock(o.m);
+  o.c.erase(std::remove(o.c.begin(), o.c.end(), c), o.c.end());
+  for (auto &b : c->pool) cudaFree(b.p);
+  c->pool.clear();
 }
 
 // the generic path's workspace: the direct RHS on the line engine's passes, the adjoint RHS, the features and the
@@ -126,7 +175,7 @@ template <class T>
 T *upload(cruna_ctx *c, const std::vector<T> &v) {
   if (v.empty()) return nullptr;
   void *p = nullptr;
-  CRUNA_CUDA_CHECK(cudaMalloc(&p, v.size() * sizeof(T)));
+  CRUNA_CUDA_CHECK(device_malloc(&p, v.size() * sizeof(T)));
   c->allocations.push_back(p);
   CRUNA_CUDA_CHECK(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
   return static_cast<T *>(p);
@@ -537,7 +586,7 @@ int cruna_init(const cruna_config *cfg, const double *bc_table, int nbc, cruna_c
     for (int i : {1, 2, 3, 5}) c->st[i] = dalloc(c, (size_t)N5(c));
     if (c->has_q_bc) c->st[4] = dalloc(c, (size_t)N5(c));
     void *fl = nullptr;
-    CRUNA_CUDA_CHECK(cudaMalloc(&fl, sizeof(int) * 4));
+    CRUNA_CUDA_CHECK(device_malloc(&fl, sizeof(int) * 4));
     c->allocations.push_back(fl);
     c->flag = static_cast<int *>(fl);  // [0] state check, [1] a kernel's bounded wait ran out
     CRUNA_CUDA_CHECK(cudaMemsetAsync(fl, 0, sizeof(int) * 4, c->stream));
@@ -589,7 +638,7 @@ void cruna_free(cruna_ctx *c) {
     cudaEventDestroy(e.b);
   }
   for (auto e : c->prof_pool) cudaEventDestroy(e);
-  for (auto &b : c->pool) cudaFree(b.p);
+  pool_free(c);
   for (void *p : c->allocations) cudaFree(p);
   for (void *p : c->snap_pinned) cudaFreeHost(p);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -1092,10 +1141,10 @@ static int gradient_common(cruna_ctx *c, const double *q0_dev, int nsteps, int n
     CRUNA_CUDA_CHECK(cudaStreamSynchronize(c->stream));
   } catch (...) {
     cudaStreamSynchronize(c->stream);
-    for (void *q : scratch) pool_give(c, q);
+    pool_give(c, scratch);
     throw;
   }
-  for (void *q : scratch) pool_give(c, q);
+  pool_give(c, scratch);
   if (direct_steps) *direct_steps = adv;
   return CRUNA_OK;
 }
@@ -1137,10 +1186,10 @@ static int optimize_common(cruna_ctx *c, const double *q0, const cruna_objective
         try {
           J = objective_direct_impl(c, q0, nsteps, obj, sc);
         } catch (...) {
-          for (void *p : sc) pool_give(c, p);
+          pool_give(c, sc);
           throw;
         }
-        for (void *p : sc) pool_give(c, p);
+        pool_give(c, sc);
         if (J_hist) J_hist[loop - 1] = J;
         break;
       }
@@ -1148,10 +1197,10 @@ static int optimize_common(cruna_ctx *c, const double *q0, const cruna_objective
       try {
         gradient_impl(c, q0, nsteps, nsnap, obj, Jd, gf, nullptr, sc);
       } catch (...) {
-        for (void *p : sc) pool_give(c, p);
+        pool_give(c, sc);
         throw;
       }
-      for (void *p : sc) pool_give(c, p);
+      pool_give(c, sc);
       CRUNA_CUDA_CHECK(cudaMemcpyAsync(&J, Jd, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
       CRUNA_CUDA_CHECK(cudaStreamSynchronize(c->stream));
       if (J_hist) J_hist[loop - 1] = J;
@@ -1167,10 +1216,10 @@ static int optimize_common(cruna_ctx *c, const double *q0, const cruna_objective
           try {
             Js[ls] = objective_direct_impl(c, q0, nsteps, obj, s2);
           } catch (...) {
-            for (void *p : s2) pool_give(c, p);
+            pool_give(c, s2);
             throw;
           }
-          for (void *p : s2) pool_give(c, p);
+          pool_give(c, s2);
         }
         copy_state(c, f, fb, 5);                               // restore_force
         // dgesv of M c = Js, M rows (a^2, a, 1): Gaussian elimination with partial pivoting
@@ -1214,11 +1263,11 @@ static int optimize_common(cruna_ctx *c, const double *q0, const cruna_objective
     CRUNA_CUDA_CHECK(cudaStreamSynchronize(c->stream));
   } catch (...) {
     cudaStreamSynchronize(c->stream);
-    for (void *p : scratch) pool_give(c, p);
+    pool_give(c, scratch);
     point_forcing(c, saved_user);
     throw;
   }
-  for (void *p : scratch) pool_give(c, p);
+  pool_give(c, scratch);
   point_forcing(c, saved_user);
   return CRUNA_OK;
 }
@@ -1237,10 +1286,10 @@ int cruna_objective_value_dev(cruna_ctx *c, const double *q0, int nsteps, const 
     try {
       *J = objective_direct_impl(c, q0, nsteps, obj, sc);
     } catch (...) {
-      for (void *p : sc) pool_give(c, p);
+      pool_give(c, sc);
       throw;
     }
-    for (void *p : sc) pool_give(c, p);
+    pool_give(c, sc);
     return CRUNA_OK;
   });
 }

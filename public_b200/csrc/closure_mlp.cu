@@ -503,6 +503,11 @@ void ck(cudaError_t e, const char *what) {
   }
 }
 
+template <class T>
+cudaError_t dmalloc(T **p, size_t bytes) {
+  return cruna::device_malloc(reinterpret_cast<void **>(p), bytes);
+}
+
 template <class F>
 int mlp_guard(cruna_mlp *h, F &&f) {
   if (!h) return CRUNA_ERR_ARG;
@@ -547,7 +552,7 @@ void ensure_idx(cruna_mlp *h, long long n) {
   if (n <= h->idx_cap) return;
   if (h->idx) cudaFree(h->idx);
   h->idx = nullptr;
-  ck(cudaMalloc(&h->idx, sizeof(int) * n), "index buffer");
+  ck(dmalloc(&h->idx, sizeof(int) * n), "index buffer");
   h->idx_cap = n;
 }
 
@@ -609,12 +614,12 @@ int cruna_mlp_create(int device, uint64_t seed, cruna_mlp **out) {
   int rc = mlp_guard(h, [&]() -> int {
     ck(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "stream");
     const int nblk = 1024;
-    ck(cudaMalloc(&h->P, sizeof(float) * NPARAMS), "params");
-    ck(cudaMalloc(&h->m, sizeof(float) * NPARAMS), "adam m");
-    ck(cudaMalloc(&h->v, sizeof(float) * NPARAMS), "adam v");
-    ck(cudaMalloc(&h->grad, sizeof(float) * (NPARAMS + 1)), "grad");
-    ck(cudaMalloc(&h->partial, sizeof(float) * (NPARAMS + 1) * nblk), "partials");
-    ck(cudaMalloc(&h->flag, sizeof(int)), "flag");
+    ck(dmalloc(&h->P, sizeof(float) * NPARAMS), "params");
+    ck(dmalloc(&h->m, sizeof(float) * NPARAMS), "adam m");
+    ck(dmalloc(&h->v, sizeof(float) * NPARAMS), "adam v");
+    ck(dmalloc(&h->grad, sizeof(float) * (NPARAMS + 1)), "grad");
+    ck(dmalloc(&h->partial, sizeof(float) * (NPARAMS + 1) * nblk), "partials");
+    ck(dmalloc(&h->flag, sizeof(int)), "flag");
     ck(cudaMemset(h->flag, 0, sizeof(int)), "flag");
     ck(cudaMemset(h->m, 0, sizeof(float) * NPARAMS), "adam m");
     ck(cudaMemset(h->v, 0, sizeof(float) * NPARAMS), "adam v");
@@ -731,7 +736,7 @@ int cruna_mlp_train_dev(cruna_mlp *h, const float *X, const float *Y, long long 
     if (steps > h->hist_cap) {
       if (h->hist) cudaFree(h->hist);
       h->hist = nullptr;
-      ck(cudaMalloc(&h->hist, sizeof(float) * std::max(steps, 1)), "loss history");
+      ck(dmalloc(&h->hist, sizeof(float) * std::max(steps, 1)), "loss history");
       h->hist_cap = steps;
     }
     const long long per_epoch = n / batch;

@@ -197,6 +197,7 @@ struct cruna_ctx {
     bool used;
   };
   std::vector<PoolBuf> pool;       // buffers of the gradient and objective calls (pool_take, capi.cu)
+  bool pool_grown = false;         // buffers came in since the last pool_give
   std::vector<void *> snap_pinned;  // those host slots (one state each), kept for later gradient calls
   // step graphs (step_graph.cu): the cache of the current run call, or null outside one
   bool graphs_enabled = true;
@@ -282,9 +283,9 @@ void graph_step(cruna_ctx *c, int kind, const void *a, const void *b, const void
                 const std::function<void()> &body);
 double *dalloc(cruna_ctx *c, size_t count);
 void attach_factors(cruna_ctx *c, LineOp &op, const HostFactors &hf);
+cudaError_t device_malloc(void **p, size_t bytes);  // every device allocation of the library (capi.cu)
 void *pool_take(cruna_ctx *c, size_t bytes);
-void pool_give(cruna_ctx *c, void *p);
-void pool_trim(cruna_ctx *c, size_t keep);
+void pool_give(cruna_ctx *c, std::vector<void *> &bufs);
 void ensure_generic(cruna_ctx *c);
 bool use_fused(const cruna_ctx *c);
 // learned closure (closure_mlp.cu, closure_ops.cu)

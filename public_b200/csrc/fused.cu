@@ -758,7 +758,7 @@ static FusedArgs flow_args(const cruna_ctx *c) {
 static void ensure_intermediates(cruna_ctx *c, bool fp32) {
   if (c->fz) return;
   void *p = nullptr;
-  CRUNA_CUDA_CHECK(cudaMalloc(&p, (size_t)NG * c->g.N * (fp32 ? sizeof(float) : sizeof(double))));
+  CRUNA_CUDA_CHECK(device_malloc(&p, (size_t)NG * c->g.N * (fp32 ? sizeof(float) : sizeof(double))));
   c->allocations.push_back(p);
   c->fz = static_cast<double *>(p);
 }

@@ -277,7 +277,7 @@ int cruna_run_hpc(cruna_ctx *ctx, double *q_io, const cruna_hpc_opts *o, int *ns
     return CRUNA_ERR_CUDA;
   };
   cudaError_t e = cudaSetDevice(c.device);
-  if (e == cudaSuccess) e = cudaMalloc(&dq, sizeof(double) * M);
+  if (e == cudaSuccess) e = cruna::device_malloc(reinterpret_cast<void **>(&dq), sizeof(double) * M);
   if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? CRUNA_ERR_NOMEM : cuda_fail(e);
   auto store = [&](int ns, int nt, bool restartfile) -> int {
     // the device state through q_io (the caller's host array) into the snapshot file

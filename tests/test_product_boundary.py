@@ -3,6 +3,7 @@ every module (the C-ABI binding, the closure, slabs, autograd, the study scripts
 import ast
 import glob
 import os
+import re
 import subprocess
 import sys
 
@@ -32,3 +33,15 @@ def test_importing_the_package_leaves_the_oracle_unloaded():
     r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
     assert r.stdout.strip().splitlines()[-1] == "[]", r.stdout
+
+
+def test_device_memory_comes_from_one_place():
+    # device_malloc frees the idle work buffers of the contexts before an allocation fails: nothing may pass it by
+    calls = []
+    for path in sorted(glob.glob(os.path.join(ROOT, "public_b200", "csrc", "*"))):
+        with open(path) as f:
+            text = re.sub(r"//[^\n]*", "", f.read())
+        for m in re.finditer(r"\bcudaMalloc(?:Async|Managed)?\(", text):
+            at = text.rfind("\n}", 0, m.start())
+            calls.append((os.path.basename(path), text[at:m.start()].strip().lstrip("}").split("(")[0].strip()))
+    assert set(calls) == {("capi.cu", "cudaError_t device_malloc")}, calls

@@ -211,15 +211,28 @@ void ensure_reference(cruna_ctx *c) {
   CRUNA_CUDA_CHECK(cudaMemsetAsync(c->qref, 0, sizeof(double) * N5(c), c->stream));
 }
 
-// the RHS buffer st[0]: the generic path's RHS and the fused path's RHS before RHS boundary conditions
+// the RHS buffer st[0], where a step forms the RHS before the stage update: the sequence of single derivatives,
+// and RHS boundary conditions on the finished RHS
 double *rhs_buffer(cruna_ctx *c) {
   if (!c->st[0]) c->st[0] = dalloc(c, (size_t)N5(c));
   return c->st[0];
 }
+bool direct_needs_rhs(const cruna_ctx *c) {
+  if (use_fused(c)) return c->has_rhs_bc;
+  if (c->march_y_ok || c->dir_ok) return c->has_rhs_bc && !only_sponge(c);  // their last pass takes a lone sponge row
+  return true;
+}
+bool adjoint_needs_rhs(const cruna_ctx *c) {
+  if (use_fused(c)) return c->has_rhs_bc;
+  if (!c->march_y_ok) return true;
+  for (const BCRow &r : c->bc)
+    if (r.type == 100) return true;   // :518 without q: only the walls act
+  return false;
+}
 
 // time_stepper_direct (rk_o4_e.f90:17-58): q1 may alias q0
 void step_direct(cruna_ctx *c, const double *q0, double *q1) {
-  double *k = ((use_fused(c) || c->dir_ok || c->march_y_ok) && !c->has_rhs_bc) ? nullptr : rhs_buffer(c);
+  double *k = direct_needs_rhs(c) ? rhs_buffer(c) : nullptr;
   double *acc = c->st[1], *qa = c->st[2], *qb = c->st[3], *qbc = c->st[4];
   const double dt = c->cfg.dt;
   if (use_fused(c)) {
@@ -254,7 +267,7 @@ void step_direct(cruna_ctx *c, const double *q0, double *q1) {
 
 // time_stepper_adjoint (rk_o4_e.f90:62-105): dt -> -dt, q0 frozen; qs1 may alias qs0
 void step_adjoint(cruna_ctx *c, const double *qs0, const double *q0, const double *g, double *qs1) {
-  double *k = ((use_fused(c) || c->march_y_ok) && !c->has_rhs_bc) ? nullptr : rhs_buffer(c);
+  double *k = adjoint_needs_rhs(c) ? rhs_buffer(c) : nullptr;
   double *acc = c->st[1], *qa = c->st[2], *qb = c->st[3], *qbc = c->st[4];
   const double dt = -c->cfg.dt;
   halo(c, q0, 5);

@@ -1,7 +1,9 @@
-"""Work buffers kept with the context between gradient and objective calls: whatever was called before, with
-other snapshot counts, host snapshots or another context in between, a call gives the bits that a fresh context gives."""
+"""Work buffers of a context: whatever gradient or objective call ran before, with other snapshot counts, host
+snapshots or another context in between, a call gives the bits that a fresh context gives; and a step allocates no more
+than its path needs."""
 import numpy as np
 import pytest
+import torch
 
 from public_b200 import cases
 from public_b200.cruna import Cruna, Settings
@@ -35,3 +37,20 @@ def test_calls_on_one_context_match_fresh_contexts(mode):
                 ref = call(fresh)
             for a, b in zip(np.atleast_1d(got) if np.isscalar(got) else got, np.atleast_1d(ref) if np.isscalar(ref) else ref):
                 assert np.array_equal(np.asarray(a), np.asarray(b))
+
+
+def test_a_marching_run_with_a_sponge_allocates_no_rhs_buffer():
+    # 47 workspace fields and 15 intermediates; the 5 of an RHS buffer (31 MB here) would not fit the 16 MB of slack
+    n = (128, 96, 64)
+    used = []
+    for size in ((20, 40, 17), n):              # the first run loads the kernels
+        s, q = cases.mixing_layer(n=size)
+        with Cruna(Settings.from_dict(s), qref=q) as c:
+            qd, qs = torch.from_numpy(np.ascontiguousarray(q.T)).cuda(), torch.zeros(q.size, dtype=torch.float64, device="cuda")
+            torch.cuda.synchronize()
+            before = torch.cuda.mem_get_info()[0]
+            c.step_direct_dev(qd.data_ptr(), qd.data_ptr())
+            c.step_adjoint_dev(qs.data_ptr(), qd.data_ptr(), None, qs.data_ptr())
+            c.sync()
+            used.append(before - torch.cuda.mem_get_info()[0])
+    assert used[-1] <= 62 * 8 * n[0] * n[1] * n[2] + (16 << 20), used

@@ -121,9 +121,11 @@ static void pool_free(cruna_ctx *c) {
 }
 
 // the generic path's workspace: the direct RHS on the line engine's passes, the adjoint RHS, the features and the
-// discrete adjoint stay below grad p's last field; only the direct RHS as single derivatives uses the rest
+// discrete adjoint stay below kShortFields; only the direct RHS as single derivatives uses the rest
 void ensure_generic(cruna_ctx *c) {
-  if (!c->tmp) c->tmp = dalloc(c, (size_t)c->g.N * (c->dir_ok || c->march_y_ok ? F_PZ + 1 : kGenericFields));
+  if (c->tmp) return;
+  const int fields = c->march_y_ok ? kShortFields + 2 : (c->dir_ok ? kShortFields : kGenericFields);
+  c->tmp = dalloc(c, (size_t)c->g.N * fields);
 }
 
 bool use_fused(const cruna_ctx *c) { return c->fused_ok && !c->force_generic; }
@@ -283,6 +285,7 @@ void step_adjoint(cruna_ctx *c, const double *qs0, const double *q0, const doubl
     return;
   }
   ensure_generic(c);
+  if (c->march_y_ok) adjoint_freeze_march_y(c, q0);
   halo(c, qs0, 5);
   stage_adjoint_generic(c, qs0, q0, g, k, qbc, 1, qs0, acc, qa, dt);
   halo(c, qa, 5);

@@ -236,6 +236,7 @@ void dir_viscous(cruna_ctx *c, int d, const double *t1, const double *t2, const 
 bool march_y_supported(const cruna_ctx *c);
 void rhs_direct_march_y(cruna_ctx *c, const double *q, double *rhs, double *qbc_scratch, int bc_mask, int stage,
                         const double *q0, double *acc, double *qnext, double dt);
+void adjoint_freeze_march_y(cruna_ctx *c, const double *q);  // once before the stages on the frozen state q
 void rhs_adjoint_march_y(cruna_ctx *c, const double *qs, const double *q, const double *g, double *rhs,
                          double *qsbc_scratch, int stage, const double *qs0, double *acc, double *qnext, double dt);
 // one RK stage of the generic path: its RHS and the stage update

@@ -35,7 +35,7 @@ struct AdjArgs {
   const double *q0;
   double *acc;
   double *qnext;
-  const double *yd;    // YX: the y derivatives of p, qs1..qs5 and v qs5, from the line engine
+  const double *yd, *py;  // YX: the y derivatives of qs1..qs5 and v qs5, and of p, from the line engine
 };
 
 // per-direction contribution in the reference's order (ns_rho_rhou_p.f90:317-370 / 386-440 / 456-509)
@@ -176,7 +176,8 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
     if (inside) {
       if constexpr (YX) {
 #pragma unroll
-        for (int v = 0; v < 7; ++v) e_y[v] = (a.yd + v * N)[opt];
+        for (int v = 0; v < 6; ++v) e_y[v] = (a.yd + v * N)[opt];
+        e_y[6] = a.py[opt];
       }
       if (a.src) {
 #pragma unroll
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(TX *TY, sizeof(T) == 4 ? 3 : 2) k_adj_pass(con
         adj_dir(0, u1, u2, u3, gpr, ir, qs5, a.gamma, A, B, Cc, D, E, Sx, P, r1, r2, r3, r4, r5);
       }
       if constexpr (YX) {
-        adj_dir(1, u1, u2, u3, gpr, ir, qs5, a.gamma, e_y[1], e_y[2], e_y[3], e_y[4], e_y[5], e_y[6], e_y[0], r1, r2, r3, r4, r5);
+        adj_dir(1, u1, u2, u3, gpr, ir, qs5, a.gamma, e_y[0], e_y[1], e_y[2], e_y[3], e_y[4], e_y[5], e_y[6], r1, r2, r3, r4, r5);
       } else {
         const double s = oy.scale;
         const double A = D1<T, R, PER>(oy, c, PW, j) * s, B = D1<T, R, PER>(oy, c + PS, PW, j) * s,
@@ -774,11 +775,22 @@ __global__ void k_adj_v(long long N, const double *__restrict__ q, double *__res
     v[p] = q[p + 2 * N] / q[p];
 }
 
-// adjoint RHS or RK stage with a compact scheme along y (march_y_supported): the y derivatives of qs1..qs5 and
-// v qs5 in one launch of the line engine, everything else in the z-marching pass.  v and the y derivative of the
-// frozen state's p are formed with the first stage of a step and stay in the workspace for the other three.
-// Mixing layer 256 x 192 x 128: the pass that also summed the y terms on the line engine took 600 us a stage,
-// the plain derivatives 240 (loop step 5.13 -> 3.56 ms).
+// what the adjoint RHS with a compact scheme along y needs of the frozen state q: v and the y derivative of p, in
+// workspace fields of their own.  Formed once before the four stages of a step, which read them.
+void adjoint_freeze_march_y(cruna_ctx *c, const double *q) {
+  const long long N = c->g.N;
+  {
+    ProfScope ps(c, "adj_freeze");
+    k_adj_v<<<(int)std::min<long long>((N + 255) / 256, 148LL * 32), 256, 0, c->stream>>>(N, q, c->tmp + F_FROZEN_V * N);
+    CRUNA_LAUNCH_CHECK(c);
+  }
+  apply_diff(c, 1, q + 4 * N, nullptr, c->tmp + F_FROZEN_PY * N, c->dx[1], 1);
+}
+
+// adjoint RHS or RK stage with a compact scheme along y (march_y_supported) after adjoint_freeze_march_y(c, q): the y
+// derivatives of qs1..qs5 and v qs5 in one launch of the line engine, everything else in the z-marching pass.
+// Mixing layer 256 x 192 x 128: a pass that also summed the y terms on the line engine took 600 us a stage, the six
+// plain derivatives 165 (loop step 5.13 -> 3.31 ms).
 void rhs_adjoint_march_y(cruna_ctx *c, const double *qs_in, const double *q, const double *g, double *rhs, double *qsbc,
                          int stage, const double *qs0, double *acc, double *qnext, double dt) {
   const double *qs = qs_in;
@@ -788,15 +800,11 @@ void rhs_adjoint_march_y(cruna_ctx *c, const double *qs_in, const double *q, con
     qs = qsbc;
   }
   const long long N = c->g.N;
-  double *v = c->tmp, *yd = v + N;
-  if (stage <= 1) {
-    k_adj_v<<<(int)std::min<long long>((N + 255) / 256, 148LL * 32), 256, 0, c->stream>>>(N, q, v);
-    CRUNA_LAUNCH_CHECK(c);
-    apply_diff(c, 1, q + 4 * N, nullptr, yd, c->dx[1], 1);
-  }
+  const double *v = c->tmp + F_FROZEN_V * N;
+  double *yd = c->tmp;
   FieldSet fs;
-  for (int f = 0; f < 5; ++f) fs.add(qs + f * N, nullptr, yd + (1 + f) * N);
-  fs.add(qs + 4 * N, v, yd + 6 * N);
+  for (int f = 0; f < 5; ++f) fs.add(qs + f * N, nullptr, yd + f * N);
+  fs.add(qs + 4 * N, v, yd + 5 * N);
   apply_diff_set(c, 1, fs, c->dx[1]);
   bool walls = false;                                              // :518 without q: only the walls act
   for (const BCRow &b : c->bc) walls = walls || b.type == 100;
@@ -813,6 +821,7 @@ void rhs_adjoint_march_y(cruna_ctx *c, const double *qs_in, const double *q, con
   a.acc = acc;
   a.qnext = qnext;
   a.yd = yd;
+  a.py = c->tmp + F_FROZEN_PY * N;
   a.stage = walls ? 0 : stage;
   a.rhs = a.stage == 0 ? rhs : nullptr;
   constexpr int R = 4;

@@ -1347,6 +1347,7 @@ void stage_adjoint_generic(cruna_ctx *c, const double *qs, const double *q, cons
 void rhs_adjoint_generic(cruna_ctx *c, const double *qs_in, const double *q, const double *g, double *rhs,
                          double *qsbc) {
   if (c->march_y_ok) {
+    adjoint_freeze_march_y(c, q);
     rhs_adjoint_march_y(c, qs_in, q, g, rhs, qsbc, 0, nullptr, nullptr, nullptr, 0.0);
     return;
   }

@@ -157,5 +157,8 @@ enum GenericField {
   F_EX, F_EY, F_EZ, F_QX, F_QY, F_QZ,
   kGenericFields
 };
+// fields of a workspace without the ones that only the direct RHS as single derivatives uses; two more of the
+// adjoint's frozen state follow where a compact scheme along y marches in x and z (adjoint_freeze_march_y)
+constexpr int kShortFields = F_PZ + 1, F_FROZEN_V = kShortFields, F_FROZEN_PY = kShortFields + 1;
 
 }  // namespace cruna

@@ -648,9 +648,11 @@ void launch_passes(cruna_ctx *c, FusedArgs &a) {
                                             (int)smem_g_cl<T, R>()));
       cl_configured = true;
     }
-    // two blocks an SM (registers and shared memory; the occupancy query does not report them for this kernel): 64^3
-    // runs 256 blocks of 8 planes in place of 128 of 16
-    a.kc = z_chunk_balanced(c->g.n3, bx * by, 2, sms, R, nz);
+    // blocks an SM from the launch bounds and the shared memory: the occupancy query answers 1 for this kernel (it
+    // allocates TMEM), but two run side by side in FP64 -- 64^3 as 256 blocks of 8 planes takes 90 us, as 128 of 16
+    // 122, which one block an SM could not do
+    const int res_cl = std::min(sizeof(T) == 4 ? 3 : 2, (int)(233472 / (smem_g_cl<T, R>() + 1024)));
+    a.kc = z_chunk_balanced(c->g.n3, bx * by, res_cl, sms, R, nz);
     ProfScope ps(c, "pass_g_closure");
     k_pass_g<T, R, PER, true><<<dim3(bx, by, nz), dim3(TX, TY), smem_g_cl<T, R>(), c->stream>>>(a);
     CRUNA_LAUNCH_CHECK(c);

@@ -666,7 +666,7 @@ void apply_filter(cruna_ctx *c, int dir, double *q, double *scratch, int nfields
 // boundary kernels
 // ------------------------------------------------------------------------------------------------
 
-// characteristic_q_k1d (src/boundaries/nonreflecting.f90:46-137) -- aim from `aim` at p + aim_off (type 200)
+// characteristic_q_k1d (src/boundaries/nonreflecting.f90:46-137) -- aim from `aim` at p + aim_off
 __global__ void k_char_q(Box b, Grid g, double k1, double k2, double k3, double gamma, double *q,
                          const double *aim, long long aim_off) {
   const long long tot = b.count();
@@ -726,7 +726,9 @@ __global__ void k_char_rhs(Box b, Grid g, double k1, double k2, double k3, doubl
 
 // Consecutive type-201 rows in one launch (a launch costs about 5 us whatever the box): row = blockIdx.y.  Rows
 // apply in table order where boxes overlap (edges and corners): the first row that holds a point does all of
-// them there, one after another; the treatment only touches its own point.
+// them there, one after another; the treatment only touches its own point.  A row by itself, or of more than 2^19
+// points (where the other boxes' tests cost more than a launch: 553,000 points beside two of 58,000, 51 against 46 us),
+// runs as k_char_q / k_char_qs.
 struct CharRows {
   static constexpr int kMax = 8;
   int n = 0;
@@ -765,12 +767,16 @@ __global__ void k_char_rows(const __grid_constant__ CharRows rows, Grid g, doubl
   }
 }
 
-// the type-201 rows from position at on (as many as fit one launch); returns the position after them
+static bool joins(const cruna_ctx *c, size_t at) {
+  return at < c->bc.size() && c->bc[at].type == 201 && box_of(c->bc[at]).count() <= 1 << 19;
+}
+
+// the joining type-201 rows from position at on (as many as fit one launch); returns the position after them
 template <bool ADJ>
 static size_t launch_char_rows(cruna_ctx *c, size_t at, double *q, const double *aim) {
   CharRows rows;
   int blocks = 1;
-  for (; at < c->bc.size() && c->bc[at].type == 201 && rows.n < CharRows::kMax; ++at) {
+  for (; joins(c, at) && rows.n < CharRows::kMax; ++at) {
     rows.box[rows.n] = box_of(c->bc[at]);
     for (int d = 0; d < 3; ++d) rows.k[rows.n][d] = c->bc[at].k[d];
     blocks = std::max(blocks, nblocks(rows.box[rows.n].count()));
@@ -931,15 +937,15 @@ void bc_q(cruna_ctx *c, double *q, int outside) {
   ProfScope ps(c, "boundary");
   for (size_t at = 0; at < c->bc.size(); ++at) {
     const BCRow &r = c->bc[at];
-    if (r.type == 201) {
+    if (joins(c, at) && joins(c, at + 1)) {
       at = launch_char_rows<false>(c, at, q, c->qref) - 1;
       continue;
     }
     Box b = box_of(r);
     const int blocks = nblocks(b.count());
-    if (r.type == 200) {
-      k_char_q<<<blocks, kThreads, 0, c->stream>>>(b, c->g, r.k[0], r.k[1], r.k[2], c->cfg.gamma, q, q,
-                                                   offset_of(c, r.shift));
+    if (r.type == 200 || r.type == 201) {
+      k_char_q<<<blocks, kThreads, 0, c->stream>>>(b, c->g, r.k[0], r.k[1], r.k[2], c->cfg.gamma, q,
+                                                   r.type == 200 ? q : c->qref, r.type == 200 ? offset_of(c, r.shift) : 0);
       CRUNA_LAUNCH_CHECK(c);
     } else if (r.type == 401) {
       k_sponge<<<nblocks(c->g.N), kThreads, 0, c->stream>>>(1, c->g, c->sponge, c->cfg.gamma, q, nullptr,
@@ -957,14 +963,14 @@ void bc_qs(cruna_ctx *c, double *qs, const double *q, int outside) {
   ProfScope ps(c, "boundary");
   for (size_t at = 0; at < c->bc.size(); ++at) {
     const BCRow &r = c->bc[at];
-    if (r.type == 201) {
+    if (joins(c, at) && joins(c, at + 1)) {
       at = launch_char_rows<true>(c, at, qs, q) - 1;
       continue;
     }
     Box b = box_of(r);
     const int blocks = nblocks(b.count());
-    if (r.type == 200) {
-      const long long off = offset_of(c, r.shift);
+    if (r.type == 200 || r.type == 201) {
+      const long long off = r.type == 200 ? offset_of(c, r.shift) : 0;
       k_char_qs<<<blocks, kThreads, 0, c->stream>>>(b, c->g, r.k[0], r.k[1], r.k[2], c->cfg.gamma, qs, q,
                                                     off);
       CRUNA_LAUNCH_CHECK(c);

@@ -122,3 +122,33 @@ def test_long_lines_leave_the_line_engine_on_many_lines(n, d, diff, filt):
         assert np.max(np.abs(got["dx"][..., v] - ref)) < 1e-12 * np.max(np.abs(ref)), v
     ref = O.filter_dir(cfg, d, f)
     assert np.max(np.abs(got["filt"] - ref)) < 1e-12 * np.max(np.abs(ref))
+
+
+def test_type_201_rows_join_in_runs_and_keep_table_order():
+    # overlapping faces (joined, more than one launch holds), a box of more than 2^19 points and a row by itself,
+    # none of which commute: to 1e-12 relative L2 per variable; launches: 8 + 1, the box, the last row
+    n = (96, 80, 72)
+    full = [1, n[0], 1, n[1], 1, n[2]]
+    faces = []
+    for d in range(3):
+        for end in (1, n[d]):
+            box, k = list(full), [0.0, 0.0, 0.0]
+            box[2 * d] = box[2 * d + 1] = end
+            k[d] = -1.0 if end == 1 else 1.0
+            faces.append([201, *box, *k])
+    bc = np.array(faces + faces[:3] + [[201, *full, 0, 1, 0], faces[2]], dtype=float)
+    q = cases.smooth_random_state(n, seed=3)
+    rng = np.random.default_rng(4)
+    ref = np.asfortranarray(q * (1.0 + 1e-2 * rng.standard_normal(q.shape)))
+    qs = np.asfortranarray(0.1 * rng.standard_normal(q.shape))
+    s = dict(BASE, n=n, diff=("o4_e_c_o",) * 3, bc=bc)
+    S = O.Solver(O.Config(**s), qref=ref)
+    with Cruna(Settings(**s), qref=ref) as c:
+        before = c.launches
+        got = c.set_boundary_condition_q(q)
+        assert c.launches - before == 4
+        got_s = c.set_boundary_condition_qs(qs, q)
+        assert c.launches - before == 8
+    for a, b in ((got, S.set_boundary_condition_q(q)), (got_s, S.set_boundary_condition_qs(qs, q))):
+        for v in range(5):
+            assert np.linalg.norm(a[..., v] - b[..., v]) <= 1e-12 * np.linalg.norm(b[..., v]), v

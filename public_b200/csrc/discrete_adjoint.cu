@@ -670,16 +670,22 @@ void interior_vjp(cruna_ctx *c, const double *qb, const double *lam, double *mu,
     diff_T(c, d, lam, c->tmp + (long long)slots[d] * N, c->dx[d], 5, 0);
     dirs.ratio[d] = diff_scale(c, d, hT[d]) / diff_scale(c, d, c->dx[d]);
   }
-  k_vjp_point<<<blocks, kThreads, 0, c->stream>>>(N, dirs, gamma, cp_pr, qb, lam, c->tmp, w);
-  CRUNA_LAUNCH_CHECK(c);
+  {
+    ProfScope ps(c, "vjp_point");
+    k_vjp_point<<<blocks, kThreads, 0, c->stream>>>(N, dirs, gamma, cp_pr, qb, lam, c->tmp, w);
+    CRUNA_LAUNCH_CHECK(c);
+  }
   for (int d = 0; d < 3; ++d) {
     if (!live[d]) continue;
     diff_T(c, d, Wf(V_B + d), Wf(V_PB), c->dx[d], 1, 1);      // grad p
     diff_T(c, d, Wf(V_GB + 3 * d), Wf(V_UB), c->dx[d], 3, 1);  // grad u, v, w along d
     diff_T(c, d, Wf(V_TGB + d), Wf(V_TB), hT[d], 1, 1);        // grad T
   }
-  k_vjp_final<<<blocks, kThreads, 0, c->stream>>>(N, c->cfg.W / c->cfg.R, qb, c->tmp, w, mu, lam_q);
-  CRUNA_LAUNCH_CHECK(c);
+  {
+    ProfScope ps(c, "vjp_point");
+    k_vjp_final<<<blocks, kThreads, 0, c->stream>>>(N, c->cfg.W / c->cfg.R, qb, c->tmp, w, mu, lam_q);
+    CRUNA_LAUNCH_CHECK(c);
+  }
 }
 
 __global__ void k_lin2(long long M, double a, const double *__restrict__ x, double b, const double *__restrict__ y,

@@ -828,7 +828,8 @@ void rhs_direct_fused(cruna_ctx *c, const double *q_in, double *rhs, int stage, 
 // ------------------------------------------------------------------------------------------------
 // compact schemes along y between explicit o8 ones along x and z: the z-marching passes for x and z, the
 // line engine's passes for y (dir_passes.cu).  684 bytes a point and RK stage (y flux pass 112, pass G 232, y
-// viscous pass 64, pass D 276) against 1040 with every direction on the line engine.
+// viscous pass 96, pass D 244; a sponge row 5 to 80 more where its shape is not zero) against 1040 with every
+// direction on the line engine.
 // ------------------------------------------------------------------------------------------------
 bool march_y_supported(const cruna_ctx *c) {
   for (int d : {0, 2}) {

@@ -1204,8 +1204,11 @@ void rhs_direct_generic(cruna_ctx *c, const double *q_in, double *rhs, double *q
   }
   const double *ru = q + N, *rv = q + 2 * N, *rw = q + 3 * N, *pp = q + 4 * N;
   const int blocks = (int)std::min<long long>(nblocks(N), 148LL * 32);
-  k_prim<<<blocks, kThreads, 0, c->stream>>>(N, q, t, c->cfg.W / c->cfg.R);
-  CRUNA_LAUNCH_CHECK(c);
+  {
+    ProfScope ps(c, "generic_point");
+    k_prim<<<blocks, kThreads, 0, c->stream>>>(N, q, t, c->cfg.W / c->cfg.R);
+    CRUNA_LAUNCH_CHECK(c);
+  }
   const double *dx = c->dx;
   // velocity gradients (:102-112), the three components of one direction in one launch
   for (int d = 0; d < 3; ++d) {
@@ -1216,10 +1219,13 @@ void rhs_direct_generic(cruna_ctx *c, const double *q_in, double *rhs, double *q
   // temperature gradient for the heat flux (:189-191), h absent unless heat_flux_dx
   for (int d = 0; d < 3; ++d)
     apply_diff(c, d, F(F_T), nullptr, F(F_TX + d), c->cfg.heat_flux_dx ? dx[d] : 1.0, 1);
-  k_visc<<<blocks, kThreads, 0, c->stream>>>(N, t, c->cfg.mu0, c->cfg.T0,
-                                             c->cfg.gamma * (c->cfg.R / c->cfg.W) / (c->cfg.gamma - 1.0) /
-                                                 c->cfg.Pr);
-  CRUNA_LAUNCH_CHECK(c);
+  {
+    ProfScope ps(c, "generic_point");
+    k_visc<<<blocks, kThreads, 0, c->stream>>>(N, t, c->cfg.mu0, c->cfg.T0,
+                                               c->cfg.gamma * (c->cfg.R / c->cfg.W) / (c->cfg.gamma - 1.0) /
+                                                   c->cfg.Pr);
+    CRUNA_LAUNCH_CHECK(c);
+  }
   // mass (:131-133)
   apply_diff(c, 0, ru, nullptr, F(F_M1), dx[0], 1);
   apply_diff(c, 1, rv, nullptr, F(F_M2), dx[1], 1);
@@ -1243,8 +1249,11 @@ void rhs_direct_generic(cruna_ctx *c, const double *q_in, double *rhs, double *q
   for (int d = 0; d < 3; ++d) apply_diff(c, d, pp, F(F_U1 + d), F(F_EX + d), dx[d], 1);
   for (int d = 0; d < 3; ++d)
     apply_diff(c, d, F(F_HX + d), nullptr, F(F_QX + d), c->cfg.heat_flux_dx ? dx[d] : 1.0, 1);
-  k_assemble<<<blocks, kThreads, 0, c->stream>>>(N, t, rhs, c->cfg.gamma, c->force);
-  CRUNA_LAUNCH_CHECK(c);
+  {
+    ProfScope ps(c, "generic_point");
+    k_assemble<<<blocks, kThreads, 0, c->stream>>>(N, t, rhs, c->cfg.gamma, c->force);
+    CRUNA_LAUNCH_CHECK(c);
+  }
   if (c->has_rhs_bc && (bc_mask & 2)) bc_rhs(c, rhs, q);  // :218
 }
 
@@ -1255,8 +1264,11 @@ void generic_forward_gradients(cruna_ctx *c, const double *q) {
   double *t = c->tmp;
   auto F = [&](int f) { return t + (long long)f * N; };
   const int blocks = (int)std::min<long long>(nblocks(N), 148LL * 32);
-  k_prim<<<blocks, kThreads, 0, c->stream>>>(N, q, t, c->cfg.W / c->cfg.R);
-  CRUNA_LAUNCH_CHECK(c);
+  {
+    ProfScope ps(c, "generic_point");
+    k_prim<<<blocks, kThreads, 0, c->stream>>>(N, q, t, c->cfg.W / c->cfg.R);
+    CRUNA_LAUNCH_CHECK(c);
+  }
   const double *dx = c->dx;
   for (int d = 0; d < 3; ++d) {
     FieldSet fs;
@@ -1265,10 +1277,13 @@ void generic_forward_gradients(cruna_ctx *c, const double *q) {
   }
   for (int d = 0; d < 3; ++d)
     apply_diff(c, d, F(F_T), nullptr, F(F_TX + d), c->cfg.heat_flux_dx ? dx[d] : 1.0, 1);
-  k_visc<<<blocks, kThreads, 0, c->stream>>>(N, t, c->cfg.mu0, c->cfg.T0,
-                                             c->cfg.gamma * (c->cfg.R / c->cfg.W) / (c->cfg.gamma - 1.0) /
-                                                 c->cfg.Pr);
-  CRUNA_LAUNCH_CHECK(c);
+  {
+    ProfScope ps(c, "generic_point");
+    k_visc<<<blocks, kThreads, 0, c->stream>>>(N, t, c->cfg.mu0, c->cfg.T0,
+                                               c->cfg.gamma * (c->cfg.R / c->cfg.W) / (c->cfg.gamma - 1.0) /
+                                                   c->cfg.Pr);
+    CRUNA_LAUNCH_CHECK(c);
+  }
   for (int v = 0; v < 3; ++v) apply_diff(c, v, q + 4 * N, nullptr, F(F_PX + 7 * v), dx[v], 1);
 }
 
@@ -1367,14 +1382,20 @@ void rhs_adjoint_generic(cruna_ctx *c, const double *qs_in, const double *q, con
     qs = qsbc;
   }
   const int blocks = (int)std::min<long long>(nblocks(N), 148LL * 32);
-  k_adj_prim<<<blocks, kThreads, 0, c->stream>>>(N, q, t, c->cfg.gamma);
-  CRUNA_LAUNCH_CHECK(c);
+  {
+    ProfScope ps(c, "adjoint_point");
+    k_adj_prim<<<blocks, kThreads, 0, c->stream>>>(N, q, t, c->cfg.gamma);
+    CRUNA_LAUNCH_CHECK(c);
+  }
   for (int d = 0; d < 3; ++d) {
     apply_diff(c, d, qs, nullptr, F(A_D0), c->dx[d], 5);                       // 5 fields at once
     apply_diff(c, d, qs + 4 * N, F(A_U1 + d), F(A_S), c->dx[d], 1);            // D_d(u_d*qs5)
     apply_diff(c, d, q + 4 * N, nullptr, F(A_P), c->dx[d], 1);                 // D_d p
-    k_adj_dir<<<blocks, kThreads, 0, c->stream>>>(N, d, d == 0, t, qs, rhs, c->cfg.gamma);
-    CRUNA_LAUNCH_CHECK(c);
+    {
+      ProfScope ps(c, "adjoint_point");
+      k_adj_dir<<<blocks, kThreads, 0, c->stream>>>(N, d, d == 0, t, qs, rhs, c->cfg.gamma);
+      CRUNA_LAUNCH_CHECK(c);
+    }
   }
   if (g) add_fields(c, rhs, g, 5 * N);                                         // :512
   if (c->has_rhs_bc) bc_rhss(c, rhs, qs, nullptr);                             // :518 (without q)

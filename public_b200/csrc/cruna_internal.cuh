@@ -21,7 +21,7 @@ constexpr int kMaxR = 6;        // largest interior half-width (o10 filter: 5)
 constexpr int kMaxRows = 5;     // largest number of explicit boundary rows at one end
 constexpr int kMaxRowW = 12;    // widest boundary row (o10 filter: 11 points)
 constexpr int kLineL = 16;      // points of a line held by one thread of the line engine (lines.cuh)
-constexpr int kLineEngineN = 368; // up to here a compact operator always runs on the engine (line_route, ops.cu)
+constexpr int kLineEngineN = 208; // up to here a compact operator always runs on the engine (line_route, ops.cu)
 constexpr int kLineMaxN = 2048; // longest line of the line engine: its row table takes 48 n bytes of shared memory
 
 enum OpKind { OP_ZERO = 0, OP_COPY = 1, OP_STENCIL = 2 };

@@ -491,7 +491,7 @@ static bool stencil_fast(const cruna_ctx *c, const LineOp &op) { return fast_ok(
 // With a table, a launch of enough lines leaves the engine where its blocks hold few lines (line_group): four from
 // 385 points on, two from 769, one from 1537.  Along y and z a warp then uses 32 bytes of a sector or less, and one thread
 // per line, whose time hardly depends on the number of lines, is faster once they fill the SMs.  Five fields, lines a
-// field, o6 derivative, engine / per line in us (384 points, open, z, 16384 lines: 189 / 175):
+// field, o6 derivative, engine / per line in us:
 //   open      n = 448: 4096 lines 100 / 112, 8192 179 / 141;  n = 1024: 1024 lines 141 / 174, 2048 243 / 212, 8192 891 / 308
 //   periodic  (a sweep more) n = 640: 16384 lines 489 / 567;  n = 1024: 1024 lines 128 / 210, 4096 414 / 341, 8192 784 / 436
 // Along x past 1536 points one block an SM is left, and stencil and k_line_solve are faster on many lines:
@@ -504,17 +504,25 @@ static LineRoute line_route(const cruna_ctx *c, const LineOp &op, int dir, int n
   const bool per_line = op.dl && dir > 0 && n >= 4 && n <= kPerLineMaxN;
   if (op.tab && line_grid_ok(c->g)) {
     const bool p = op.cyclic;
-    if (per_line && (n > 768 ? lines >= (p ? 16384 : 10240) : n > kLineEngineN && !p && lines >= 32768)) return ROUTE_PER_LINE;
-    return op.dl && dir == 0 && n > 1536 && lines >= (n > 1792 ? 12288 : (p ? 40960 : 20480)) ? ROUTE_GENERAL : ROUTE_ENGINE;
+    if (per_line && (n > 768 ? lines >= (p ? 16384 : 10240) : n > 384 && !p && lines >= 32768)) return ROUTE_PER_LINE;
+    return op.dl && dir == 0 && n > 1536 && lines >= (n > 1792 ? (p ? 12288 : 10240) : (p ? 40960 : 20480)) ? ROUTE_GENERAL : ROUTE_ENGINE;
   }
   return per_line ? ROUTE_PER_LINE : ROUTE_GENERAL;
 }
 
 // the route of the explicit part and the solve together: the engine and the per-line kernel take every scheme of
-// the tables above (derivatives of radius 1 and 2, filters of radius 1 to 5)
+// the tables above (derivatives of radius 1 and 2, filters of radius 1 to 5).  Where a block's lines leave it short of
+// threads, at eight lines from 209 points on and at four from 385, the operators whose windows or closure rows cost the
+// engine most are faster per line on large grids.  48 M points, five fields, engine / per line in us: o10 filter n = 192
+// 1935 / 2137, 224 2449 / 2112, 352 2551 / 2094; o8 filter 224 2119 / 1994 (12 M points, 256: 507 / 543); open o6 derivative 192 1047 / 1224, 288
+// 1473 / 1265, 384 1288 / 1267; periodic o6 derivative 384 1297 / 1779, 400 2226 / 1789; but o6 filter 384 1673 / 1894.
 static LineRoute compact_route(const cruna_ctx *c, const LineOp &op, int dir, int nfields) {
   if (op.kind != OP_STENCIL || !op.solve || op.r > (op.antisym ? 2 : 5)) return ROUTE_GENERAL;
-  const LineRoute r = line_route(c, op, dir, nfields);
+  LineRoute r = line_route(c, op, dir, nfields);
+  if (r == ROUTE_ENGINE && op.dl && dir > 0 && (c->g.N / op.n) * nfields >= (op.r == 4 ? 524288 : 131072)) {
+    const bool wide = op.antisym ? op.r == 2 : op.r >= 4;
+    if (op.cyclic ? op.antisym && op.n > 384 && op.n <= 512 : wide && op.n > kLineEngineN && op.n <= 384) r = ROUTE_PER_LINE;
+  }
   return r == ROUTE_PER_LINE && !fast_ok(op) ? ROUTE_GENERAL : r;
 }
 
@@ -600,13 +608,16 @@ static void launch_compact(cruna_ctx *c, LineRoute route, const LineOp &op, int 
 }
 
 // Dx_d of each field of a set (f1, or f1*f2 when every f2 is given), all with the same spacing h, in one
-// launch; the fallbacks take one apply_diff per field
+// launch; the fallbacks take one apply_diff per field, and compact operators on lines over 384 points where one field
+// alone leaves the engine (six fields of
+// 256 x 384 x 128 along y: one launch of the engine about 410 us, field by field 6 x 120)
 void apply_diff_set(cruna_ctx *c, int dir, const FieldSet &fs, double h) {
   const LineOp &op = c->dop[dir];
   const double scale = 1.0 / (h * op.div);
   bool uniform = true;
   for (int k = 1; k < fs.n; ++k) uniform = uniform && ((fs.f2[k] != nullptr) == (fs.f2[0] != nullptr));
-  if (compact_route(c, op, dir, 1) == ROUTE_ENGINE) {
+  const LineRoute route = compact_route(c, op, dir, 1);
+  if (route == ROUTE_ENGINE || (op.tab && route == ROUTE_PER_LINE && op.n <= 384)) {
     launch_engine_set(c, op, dir, fs, scale);
   } else if (uniform && !op.solve && stencil_fast(c, op)) {
     launch_stencil_set(c, op, dir, fs, scale, 1.0);

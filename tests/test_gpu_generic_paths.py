@@ -102,6 +102,7 @@ def test_filters_beyond_diagonal_dominance_run_one_kernel_along_y_and_z(scheme, 
 
 
 @pytest.mark.parametrize("n, d, diff, filt", [
+    ((256, 209, 103), 1, "o6_i_c_o", "o10_i_c_o"), ((128, 390, 205), 1, "o6_i_c_p", "o6_i_c_p"),
     ((64, 400, 103), 1, "o6_i_c_o", "o10_i_c_o"), ((64, 32, 800), 2, "o6_i_c_o", "o6_i_c_o"),
     ((64, 800, 52), 1, "o6_i_c_p", "o6_i_c_p"), ((64, 1024, 32), 1, "o4_i_c_o_pade", "o2_i_c_o"),
     ((1800, 50, 50), 0, "o6_i_c_o", "o10_i_c_o")])

@@ -54,7 +54,8 @@ MIXED = [(33, 9, 18), (17, 16, 15)]                  # o8 along x or y beside co
 @pytest.mark.parametrize("n, diff", [(n, d) for n in LONG for d in (("o4_e_c_o", "o8_e_c_p", "o4_e_c_p"),
                                                                     ("o6_i_c_p", "o6_i_c_o", "o4_i_c_p_pade"))]
                          + [(n, d) for n in MIXED for d in (("o8_e_c_p", "o6_i_c_o", "o6_i_c_p"),
-                                                            ("o6_i_c_p", "o8_e_c_p", "o6_i_c_o"))])
+                                                            ("o6_i_c_p", "o8_e_c_p", "o6_i_c_o"))]
+                         + [(n, ("o8_e_c_p", "o6_i_c_o", "o8_e_c_p")) for n in ((2051, 9, 8), (8, 9, 2051))])
 def test_rhs_and_steps_against_the_oracle(n, diff):
     # RHS to 1e-12 relative L2 per variable plus 1e-13 max|q| / dx (one-sided closure rows), a step to dt times the latter
     q = cases.smooth_random_state(n, seed=5)
@@ -104,7 +105,8 @@ def test_filters_beyond_diagonal_dominance_run_one_kernel_along_y_and_z(scheme, 
 @pytest.mark.parametrize("n, d, diff, filt", [
     ((256, 209, 103), 1, "o6_i_c_o", "o10_i_c_o"), ((128, 390, 205), 1, "o6_i_c_p", "o6_i_c_p"),
     ((64, 400, 103), 1, "o6_i_c_o", "o10_i_c_o"), ((64, 32, 800), 2, "o6_i_c_o", "o6_i_c_o"),
-    ((64, 800, 52), 1, "o6_i_c_p", "o6_i_c_p"), ((64, 1024, 32), 1, "o4_i_c_o_pade", "o2_i_c_o"),
+    ((64, 800, 52), 1, "o6_i_c_p", "o6_i_c_p"), ((64, 1024, 52), 1, "o4_i_c_o_pade", "o2_i_c_o"),
+    ((64, 32, 900), 2, "o4_i_c_p_pade", "o8_i_c_o"), ((64, 800, 32), 1, "o4_i_c_o_pade", "o4_i_c_o"),
     ((1800, 50, 50), 0, "o6_i_c_o", "o10_i_c_o")])
 def test_long_lines_leave_the_line_engine_on_many_lines(n, d, diff, filt):
     # five fields at the sizes where the rule changes: to 1e-12 of the field maximum, as the operator parity tests

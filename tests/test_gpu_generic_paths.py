@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from oracle import cruna_oracle as O
+from oracle import discrete_adjoint as DA
 from public_b200 import cases
 from public_b200.cruna import Cruna, Settings
 
@@ -155,3 +156,28 @@ def test_type_201_rows_join_in_runs_and_keep_table_order():
     for a, b in ((got, S.set_boundary_condition_q(q)), (got_s, S.set_boundary_condition_qs(qs, q))):
         for v in range(5):
             assert np.linalg.norm(a[..., v] - b[..., v]) <= 1e-12 * np.linalg.norm(b[..., v]), v
+
+
+def test_step_vjp_with_filters_beyond_diagonal_dominance():
+    # transposed solves with row interchanges along y and z; 1e-10 relative L2 as the discrete adjoint's other tests
+    # (the matrices' condition numbers are below 1e3 at these sizes)
+    n = (14, 15, 16)
+    s = dict(BASE, n=n, diff=("o6_i_c_p", "o6_i_c_o", "o8_e_c_p"), filt=("o6_i_c_p", "o10_i_c_o", "o6_i_c_o"), alpha=0.55,
+             di_freq=(1, 1, 1))
+    for size, scheme in zip(n, s["filt"]):
+        B = np.eye(size) + 0.55 * (np.eye(size, k=1) + np.eye(size, k=-1))
+        if scheme.endswith("p"):
+            B[0, -1] = B[-1, 0] = 0.55
+        else:
+            B[0, 1] = B[-1, -2] = 0.0
+        assert np.linalg.cond(B) < 1e3
+    q = cases.smooth_random_state(n, seed=7)
+    lam = np.asfortranarray(np.random.default_rng(9).standard_normal(q.shape))
+    ref, _ = DA.step_vjp(O.Solver(O.Config(**s)), q, lam, 1)
+    with Cruna(Settings(**s)) as c:
+        out = []
+        names = kernels(c, lambda: out.append(c.step_direct_vjp(q, lam, 1)))
+    assert {"line_solve_x", "line_solve_y", "line_solve_z"} <= names
+    for v in range(5):
+        scale = max(np.linalg.norm(ref[..., v]), 1e-3 * np.linalg.norm(ref))
+        assert np.linalg.norm(out[0][..., v] - ref[..., v]) <= 1e-10 * scale, v

@@ -329,19 +329,28 @@ void attach_factors(cruna_ctx *c, LineOp &op, const HostFactors &hf) {
   if (c->g.N < (1LL << 31) - 1 && build_line_table(op.n, hf.raw_dl, hf.raw_d, hf.raw_du,
                                                    op.cyclic ? hf.fbnorm : std::vector<double>(), tab, op.kf, op.kb)) {
     op.tab = upload(c, tab);
-    if (op.n <= kLineEngineN) return;
+    // line_route leaves the engine on no launch of less than 10240 lines (eight fields at most are common)
+    if (op.n <= kLineEngineN || c->g.N / op.n * FieldSet::kMax < 10240) return;
   }
-  std::vector<double> inv(hf.d.size());
-  for (size_t i = 0; i < hf.d.size(); ++i) inv[i] = 1.0 / hf.d[i];
-  op.dl = upload(c, hf.dl);
-  op.inv_d = upload(c, inv);
-  op.du = upload(c, hf.du);
-  op.du2 = upload(c, hf.du2);
-  op.ipiv = upload(c, hf.ipiv);
+  // one array, one upload: dl, 1 / d, du, du2, fbnorm, then the interchanges
+  const size_t n = op.n;
+  std::vector<double> f(5 * n + (n + 1) / 2, 0.0);
+  std::copy(hf.dl.begin(), hf.dl.end(), f.begin());
+  for (size_t i = 0; i < n; ++i) f[n + i] = 1.0 / hf.d[i];
+  std::copy(hf.du.begin(), hf.du.end(), f.begin() + 2 * n);
+  std::copy(hf.du2.begin(), hf.du2.end(), f.begin() + 3 * n);
+  if (op.cyclic) std::copy(hf.fbnorm.begin(), hf.fbnorm.end(), f.begin() + 4 * n);
+  std::memcpy(&f[5 * n], hf.ipiv.data(), n * sizeof(int));
+  const double *p = upload(c, f);
+  op.dl = p;
+  op.inv_d = p + n;
+  op.du = p + 2 * n;
+  op.du2 = p + 3 * n;
+  if (op.cyclic) op.fbnorm = p + 4 * n;
+  op.ipiv = reinterpret_cast<const int *>(p + 5 * n);
   op.nopiv = 1;
-  for (size_t i = 0; i + 1 < hf.ipiv.size(); ++i)
+  for (size_t i = 0; i + 1 < n; ++i)
     if (hf.ipiv[i] != (int)i + 1) op.nopiv = 0;
-  if (op.cyclic) op.fbnorm = upload(c, hf.fbnorm);
 }
 
 int prof_begin(cruna_ctx *c, const char *name) {

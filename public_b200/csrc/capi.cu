@@ -329,7 +329,7 @@ void attach_factors(cruna_ctx *c, LineOp &op, const HostFactors &hf) {
   if (c->g.N < (1LL << 31) - 1 && build_line_table(op.n, hf.raw_dl, hf.raw_d, hf.raw_du,
                                                    op.cyclic ? hf.fbnorm : std::vector<double>(), tab, op.kf, op.kb)) {
     op.tab = upload(c, tab);
-    // line_route leaves the engine on no launch of less than 10240 lines (eight fields at most are common)
+    // launches of fewer than 10240 lines stay on the engine (line_route), here of up to eight fields
     if (op.n <= kLineEngineN || c->g.N / op.n * FieldSet::kMax < 10240) return;
   }
   // one array, one upload: dl, 1 / d, du, du2, fbnorm, then the interchanges
